@@ -619,6 +619,14 @@ def _prefix_exact(c, seed):
 TOP, LONGEST = 10, 56
 
 
+def _most_frequent(count):
+    """The ids of the TOP largest counts, the lower id first among equals."""
+    n = len(count)
+    rank = np.arange(n) - count * n
+    top = np.argpartition(rank, TOP)[:TOP]
+    return top[np.argsort(rank[top])]
+
+
 def _padded(names):
     """Byte strings as rows of one array, zeros behind them."""
     return np.stack([np.frombuffer(b.ljust(LONGEST, b"\0"), np.uint8) for b in names])
@@ -665,7 +673,7 @@ def _strings_run(s):
     count, total = np.empty(n, np.int64), np.empty(n, np.int64)
     count[a["keys"][0]] = a["count"][0]  # ids number the strings by first appearance
     total[a["keys"][0]] = a["i64"][1]
-    best = np.lexsort((np.arange(n), -count))[:TOP]
+    best = _most_frequent(count)
     names = s.agg.key_strings(best)
     return {"count": count, "sum": total, "top": best, "text": _padded(names)}
 
@@ -682,7 +690,7 @@ def _strings_exact(c, seed):
     order = torch.argsort(first)
     order = order[first[order] < c["rows"]]  # the strings that occur, by first appearance
     count, total = torch.bincount(pick, minlength=d)[order], _sum_by(pick, v, d)[order]
-    best = np.lexsort((np.arange(order.numel()), -count.cpu().numpy()))[:TOP]
+    best = _most_frequent(count.cpu().numpy())
     names = [pool[poff[i]:poff[i + 1]].cpu().numpy().tobytes() for i in order.cpu().numpy()[best]]
     return {"count": count, "sum": total, "top": best, "text": _padded(names)}
 
