@@ -140,3 +140,30 @@ def test_packed_and_null_keys_route_like_partition_for(ctx):
     assert_groups_equal(_concat(owned), whole.export(), ["sum_i", "count"])
     for p in partials + [whole]:
         p.close()
+
+
+@pytest.mark.parametrize("groups", [1, 255, 1023, 1024, 1025, 2049])
+@pytest.mark.parametrize("n_parts", [1, 7, 4096])
+def test_state_rows_at_tile_edges(ctx, groups, n_parts):
+    """Group counts around the partition kernels' tile of 1024 and one to 4096 owners: every group's row
+    comes out once, in its owner's range, with its state."""
+    import torch
+    import wadjet_b200 as wg
+    from wadjet_b200.exchange import partition_for, route_hash_int
+    k = np.repeat(np.arange(groups, dtype=np.int64) * 7919 - 5, 3)
+    v = np.arange(3 * groups, dtype=np.int64)
+    a = wg.HashAggregate(ctx, [0], [wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_MAX, 1)], ndv_hint=groups)
+    a.consume(wg.Batch([wg.Column(I64, k), wg.Column(I64, v)]))
+    rows, counts = a.partition_state(n_parts)
+    lay = a.state_layout()
+    rows = rows.cpu().numpy()
+    torch.cuda.synchronize()
+    owner = partition_for(route_hash_int(rows[:, 1]), n_parts)
+    np.testing.assert_array_equal(owner, np.repeat(np.arange(n_parts), counts))
+    order = np.argsort(rows[:, 1])
+    np.testing.assert_array_equal(rows[order, 0], 0)
+    np.testing.assert_array_equal(rows[order, 1], np.arange(groups) * 7919 - 5)
+    np.testing.assert_array_equal(rows[order, 2], 3)
+    np.testing.assert_array_equal(rows[order, 1 + lay.agg_off[0]], v.reshape(-1, 3).sum(1))
+    np.testing.assert_array_equal(rows[order, 1 + lay.agg_off[1]], v.reshape(-1, 3).max(1))
+    a.close()
