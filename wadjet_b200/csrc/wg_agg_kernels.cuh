@@ -894,15 +894,32 @@ __device__ __forceinline__ void process_rows(const Plan& P, const Sh& sh, const 
   }
 }
 
+// Words [first, n) at stride `step` of an array of slots of `period` words: the
+// first `used` words of a slot from init (shared memory), the rest 0. The
+// position within the slot advances by step mod period, so a word costs a
+// compare and an add: a modulo per word, with the pattern read by divergent
+// index from the parameter bank, held a 5.2M-word table's initialisation at 50 us
+// (18 us now) and cost a 28K-word shared table about 3 us of its kernel.
+__device__ __forceinline__ void fill_pattern(unsigned long long* out, int64_t n, int period, int used,
+                                             const unsigned long long* init, int64_t first, int64_t step) {
+  int w = (int)(first % period);
+  const int adv = (int)(step % period);
+  for (int64_t i = first; i < n; i += step) {
+    out[i] = w < used ? init[w] : 0ULL;
+    w += adv;
+    if (w >= period) w -= period;
+  }
+}
+
 // Shared slot of P.smem_sw words: the layout's slot words (empty pattern),
 // then the extra float-SUM copies (+0.0).
 __device__ __forceinline__ void smem_table_init(const Plan& P, unsigned long long* sm, int S, int* s_groups) {
+  __shared__ unsigned long long s_init[WG_MAX_SLOT_WORDS];
   const int sw = P.L.slot_words, ssw = smem_stride(P);
-  for (int i = threadIdx.x; i < S * ssw; i += blockDim.x) {
-    const int w = i % ssw;
-    sm[i] = w < sw ? P.L.init[w] : 0ULL;
-  }
+  if (threadIdx.x < (unsigned)sw) s_init[threadIdx.x] = P.L.init[threadIdx.x];
   if (threadIdx.x == 0) *s_groups = 0;
+  __syncthreads();
+  fill_pattern(sm, (int64_t)S * ssw, ssw, sw, s_init, (int64_t)threadIdx.x, (int64_t)blockDim.x);
 }
 
 template <int NA>
