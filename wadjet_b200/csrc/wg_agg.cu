@@ -851,7 +851,8 @@ static void launch_pipeline_shape(const LaunchSpec& ls, cudaStream_t st) {
     launch_static_shape(ls, st);
     return;
   }
-  if (ls.P.L.n_aggs <= 4) launch_pipeline_t<4, wgd::DynShape>(ls, st);
+  if (ls.lc && ls.smem && !ls.tile) launch_lowcard(ls, st);
+  else if (ls.P.L.n_aggs <= 4) launch_pipeline_t<4, wgd::DynShape>(ls, st);
   else launch_pipeline_t<8, wgd::DynShape>(ls, st);
 }
 
@@ -1055,6 +1056,48 @@ static int str_key_col(const wg_agg* a, const wg_batch_desc* in) {
   return kc >= 0 && kc < in->ncols && is_str_type(in->cols[kc].type_id) ? kc : -1;
 }
 
+// Shared-memory launch of a plan without a compiled shape (lowcard_kernel), or
+// none (ls.smem false: the rows update the HBM table): the expected groups (or
+// the keys of a known range [glo, ghi]) must fit the key table at most 3/4
+// full beside one copy of the accumulators, and no aggregate be a DECIMAL MIN
+// or MAX (16-byte compare-and-swap updates stay in HBM). Two CTAs per SM when a
+// half of its shared memory holds them, else one; as many copies of the
+// accumulators, up to a warp's lanes, as fit.
+static void lowcard_setup(wg_agg* a, LaunchSpec& ls, int64_t expect, bool ranged, long long glo, long long ghi,
+                          bool any_dec_minmax) {
+  Ctx* ctx = a->ctx;
+  ls.smem = ls.lc = false;
+  ls.smem_bytes = 0;
+  ls.P.smem_slots = 0;
+  ls.P.gdense = 0;
+  const int kw = a->L.key_words;
+  if (any_dec_minmax || (kw > 0 && expect <= 0) || env_int("WG_AGG_SMEM", 1) == 0) return;
+  const int64_t aw = (a->L.slot_words - kw) | 1;  // an odd stride spreads the slots over the banks
+  const bool dense = ranged && kw == 1 && ghi >= glo && env_int("WG_GROUP_DENSE", 1) != 0;
+  for (int ctas = 2; ctas >= 1; --ctas) {
+    const int64_t budget = std::min<int64_t>(ctx->max_smem_optin, ctx->smem_per_sm / ctas - 1024) - 1024;
+    const int64_t key_bytes = kw == 0 || dense ? 0 : kw * 8;
+    const int64_t fit = (budget - 2 * aw * 8) / (aw * 8 + key_bytes);  // slots beside one copy
+    int64_t S = kw == 0 ? 1 : dense ? (int64_t)(ghi - glo + 1) : std::max<int64_t>(8, 2 * expect);
+    if (S > fit && !dense && kw > 0 && expect * 4 <= fit * 3) S = fit;
+    if (S > fit || S > 16384) continue;
+    int R = 32;
+    while (R > 1 && S * key_bytes + R * (S + 2) * aw * 8 > budget) R >>= 1;
+    ls.smem = ls.lc = true;
+    ls.P.smem_slots = (int32_t)S;
+    ls.P.smem_sw = (int32_t)aw;
+    ls.P.smem_rep = R;
+    ls.P.gdense = dense ? 1 : 0;
+    ls.P.gmin = glo;
+    ls.smem_bytes = (size_t)(S * key_bytes + R * (S + 2) * aw * 8);
+    ls.block = lowcard_threads(ctas);
+    // a CTA flushes up to every slot into the HBM table: at least four rows per slot
+    const int64_t rows = std::max<int64_t>(std::max<int64_t>(lowcard_rows(ls.block), 4096), 4 * S);
+    ls.grid = (unsigned)std::min<int64_t>((int64_t)ctx->sm_count * ctas, (ls.P.n_items + rows - 1) / rows);
+    return;
+  }
+}
+
 static wg_status run_device(const PipelineRun& r) {
   wg_agg* a = r.agg;
   Ctx* ctx = a->ctx;
@@ -1157,11 +1200,11 @@ static wg_status run_device(const PipelineRun& r) {
   // dense GROUP BY: the key is a join payload column whose value range is known
   // and small, or a small string dictionary's ids, so the shared table is indexed by key - min (no hashing, no key
   // compare, no insert) and holds exactly one slot per possible key
+  long long glo = 0, ghi = -1;
+  bool ranged = false;
   {
-    long long glo = 0, ghi = -1;
     const int kv = ls.P.L.key_vcol[0];
     const int npay = r.join ? join_n_payload(r.join) : 0;
-    bool ranged = false;
     if (r.join != nullptr && join_type_of(r.join) == WG_JOIN_INNER && kv >= ls.P.n_in && kv < ls.P.n_in + npay)
       ranged = join_payload_range(r.join, kv - ls.P.n_in, &glo, &ghi);
     else if (r.str_ids && kv < ls.P.n_in) {  // a string dictionary's ids: [0, its strings)
@@ -1304,9 +1347,13 @@ static wg_status run_device(const PipelineRun& r) {
     }
   }
 
-  // shared-table row counters are 32-bit: a CTA's share of the rows stays below 2^31
-  if (ls.smem && n_items / std::max<int64_t>(1, ls.grid) >= (int64_t(1) << 31)) {
+  if (!stat && !ls.tile) lowcard_setup(a, ls, expect, ranged && ghi - glo < 16384, glo, ghi, any_dec_minmax);
+
+  // shared-table row counters are 32-bit: a CTA's share of the rows (of the
+  // matches, in the kernel that walks chains) stays below 2^31
+  if (ls.smem && n_items * (ls.lc ? fan : 1) / std::max<int64_t>(1, ls.grid) >= (int64_t(1) << 31)) {
     ls.smem = false;
+    ls.lc = false;
     ls.P.smem_slots = 0;
     ls.smem_bytes = 0;
   }
@@ -1403,13 +1450,24 @@ static wg_status run_device(const PipelineRun& r) {
       WG_TRY(rebuild_table(a, a->cap * 4, a->L));
       WG_TRY(refresh_groups(a));
       const int64_t expect2 = std::max<int64_t>(a->hint, a->known_groups);
-      if (ls.smem && !ls.P.gdense && !fits(expect2, S)) { ls.smem = false; ls.P.smem_slots = 0; ls.smem_bytes = 0; }
+      if (ls.smem && !ls.P.gdense && !fits(expect2, ls.lc ? ls.P.smem_slots : S)) {
+        ls.smem = false;
+        ls.lc = false;
+        ls.P.smem_slots = 0;
+        ls.smem_bytes = 0;
+      }
       if (table_words(a, a->cap) * 8 > kSnapshotMaxBytes) break;
     }
   }
   // 3) large table: chunks that each fit, growing between chunks
   WG_TRY(refresh_groups(a));
-  if (ls.smem) { ls.smem = false; ls.P.smem_slots = 0; ls.smem_bytes = 0; if (!ls.tile) ls.grid = (unsigned)(ctx->sm_count * 4); }
+  if (ls.smem) {
+    ls.smem = ls.lc = false;
+    ls.P.smem_slots = 0;
+    ls.smem_bytes = 0;
+    if (!ls.tile) ls.grid = (unsigned)(ctx->sm_count * 4);
+    if (!stat) ls.block = wgd::DynShape::kBlock;
+  }
   int64_t done = 0;
   const int64_t min_chunk = 1 << 20;
   while (done < n_items) {

@@ -22,6 +22,7 @@ struct LaunchSpec {
   bool tile = false;          // TMA-staged tile kernel
   wgd::TileCfg cfg{};
   int vec = 0;                // compiled shapes: rows per lane of the vector kernel (0 = one-row kernel)
+  bool lc = false;            // no compiled shape, groups in shared memory: lowcard_kernel
   bool stage = false;         // vector kernel with a shared table: the self-staged variant (1024 threads, 1 CTA/SM)
 };
 
@@ -87,7 +88,7 @@ static void launch_pipeline_t(const LaunchSpec& ls, cudaStream_t st) {
     launch_vec_t<NA, Sh>(ls, st, smem);
     return;
   }
-  if constexpr (Sh::smem_ok) {
+  if constexpr (Sh::smem_ok && !std::is_same<Sh, wgd::DynShape>::value) {  // (lowcard_kernel otherwise)
     if (smem) {
       cudaFuncSetAttribute(wgd::pipeline_kernel<NA, true, Sh>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            (int)ls.smem_bytes);
@@ -101,5 +102,11 @@ static void launch_pipeline_t(const LaunchSpec& ls, cudaStream_t st) {
 
 // Launch a compiled shape (defined in wg_agg_static.cu).
 void launch_static_shape(const LaunchSpec& ls, cudaStream_t st);
+
+// The shared-memory kernel of plans without a compiled shape (wg_agg_lowcard.cu):
+// its threads per CTA, the rows a CTA takes per step, and its launch.
+int lowcard_threads(int ctas_per_sm);
+int lowcard_rows(int threads);
+void launch_lowcard(const LaunchSpec& ls, cudaStream_t st);
 
 }  // namespace wg
