@@ -153,14 +153,7 @@ wg_status read_back_i64(Ctx* ctx, const int64_t* dev, int64_t* out, int n) {
   return WG_OK;
 }
 
-static wg_status device_error_status(Ctx* ctx, int32_t h);
-
-wg_status check_device_error(Ctx* ctx) {
-  int32_t h = 0;
-  WG_CUDA_TRY(cudaMemcpyAsync(&h, ctx->dev_error, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  WG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
-  return device_error_status(ctx, h);
-}
+wg_status check_device_error(Ctx* ctx) { return read_back_checked(ctx, nullptr, nullptr, 0); }
 
 wg_status read_back_checked(Ctx* ctx, const int64_t* dev, int64_t* out, int n) {
   int32_t h = 0;
@@ -177,7 +170,7 @@ wg_status read_back_checked(Ctx* ctx, const int64_t* dev, int64_t* out, int n) {
   return device_error_status(ctx, h);
 }
 
-static wg_status device_error_status(Ctx* ctx, int32_t h) {
+wg_status device_error_status(Ctx* ctx, int32_t h) {
   if (h == WG_DERR_NONE) return WG_OK;
   WG_CUDA_TRY(cudaMemsetAsync(ctx->dev_error, 0, sizeof(int32_t), ctx->stream));
   switch (h) {

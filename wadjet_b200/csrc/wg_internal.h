@@ -144,6 +144,7 @@ void parallel_copy(void* dst, const void* src, int64_t bytes);
 wg_status ensure_device(Ctx* ctx);           // cudaSetDevice(ctx->device)
 wg_status read_back_i64(Ctx* ctx, const int64_t* dev, int64_t* out, int n);
 wg_status check_device_error(Ctx* ctx);      // reads and clears dev_error
+wg_status device_error_status(Ctx* ctx, int32_t h);  // the status of an error word read back (clears it on the device)
 // read_back_i64 and check_device_error with one wait: n values (n < 63) and
 // the error word, which fails the call when set
 wg_status read_back_checked(Ctx* ctx, const int64_t* dev, int64_t* out, int n);
