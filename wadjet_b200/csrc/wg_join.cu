@@ -40,7 +40,34 @@ struct BuildArgs {
   int32_t* err;
 };
 
+// v summed (or its maximum taken) over the CTA's threads, in thread 0; every
+// thread of the CTA calls it. One global atomic per CTA follows where one per
+// row or slot would serialise on a single word.
+template <bool MAX>
+__device__ __forceinline__ unsigned long long cta_reduce(unsigned long long v) {
+  __shared__ unsigned long long part[32];
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long w = __shfl_down_sync(WG_FULL_MASK, v, o);
+    v = MAX ? (w > v ? w : v) : v + w;
+  }
+  const int l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
+  __syncthreads();
+  if (l == 0) part[threadIdx.x >> 5] = v;
+  __syncthreads();
+  if (threadIdx.x < 32) {
+    v = l < nw ? part[l] : 0ULL;
+    for (int o = 16; o > 0; o >>= 1) {
+      const unsigned long long w = __shfl_down_sync(WG_FULL_MASK, v, o);
+      v = MAX ? (w > v ? w : v) : v + w;
+    }
+  }
+  return v;
+}
+
+// 2^20 rows on int64 keys, two per key: 89 us with an atomic per new key on the
+// distinct counter, 57 us with one per CTA.
 __global__ void join_build_kernel(const BuildArgs a) {
+  unsigned fresh = 0;  // keys this thread installed
   for (int64_t row = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; row < a.n;
        row += (int64_t)gridDim.x * blockDim.x) {
     if (is_null(a.key, row)) continue;
@@ -60,7 +87,7 @@ __global__ void join_build_kernel(const BuildArgs a) {
           unsigned long long old = atomicCAS(s + h, cur, mine);
           if (old == cur) {
             a.next[row] = head;
-            if (head == -1) atomicAdd(a.distinct, 1ULL); else *a.dup = 1;
+            if (head == -1) ++fresh; else *a.dup = 1;
             done = true;
           } else {
             cur = old;  // lost a race on this slot: re-examine it
@@ -84,7 +111,7 @@ __global__ void join_build_kernel(const BuildArgs a) {
           U128 old = cas128(s + h, cur, mine);
           if (old.lo == cur.lo && old.hi == cur.hi) {
             a.next[row] = head;
-            if (head == -1) atomicAdd(a.distinct, 1ULL); else *a.dup = 1;
+            if (head == -1) ++fresh; else *a.dup = 1;
             done = true;
           } else {
             cur = old;
@@ -99,6 +126,8 @@ __global__ void join_build_kernel(const BuildArgs a) {
       }
     }
   }
+  const unsigned long long n = cta_reduce<false>(fresh);
+  if (threadIdx.x == 0 && n) atomicAdd(a.distinct, n);
 }
 
 struct ProbeArgs {
@@ -159,38 +188,36 @@ __global__ void join_probe_emit_kernel(const ProbeArgs a) {
   }
 }
 
-// Smallest and largest non-NULL value of an integer column (the build key's,
-// to pick a sentinel that is not a key; a payload's, for dense GROUP BY).
-// Reduced per warp and per CTA, then one atomic pair per CTA.
-__global__ void key_range_kernel(DCol key, int64_t n, long long* mn, long long* mx) {
-  long long lo = LLONG_MAX, hi = LLONG_MIN;
-  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    if (is_null(key, i)) continue;
-    const long long k = ld_i64(key, i);
-    lo = k < lo ? k : lo;
+// int64 onto uint64, order kept; and a range kept as two maxima of such words,
+// {of the values, of their complements}, so an all-zero word pair is the empty range.
+__host__ __device__ __forceinline__ unsigned long long ord_i64(long long v) {
+  return (unsigned long long)v ^ 0x8000000000000000ULL;
+}
+__host__ __device__ __forceinline__ long long unord_i64(unsigned long long w) {
+  return (long long)(w ^ 0x8000000000000000ULL);
+}
+
+// Smallest and largest non-NULL value of integer columns (the build key's, to
+// pick a sentinel that is not a key; a payload's, for dense GROUP BY): column
+// blockIdx.y into words[2 * blockIdx.y], reduced per CTA first.
+struct RangeCols {
+  DCol col[1 + WG_MAX_PAYLOAD];
+  int64_t n;
+};
+__global__ void range_kernel(const __grid_constant__ RangeCols c, unsigned long long* words) {
+  const DCol& col = c.col[blockIdx.y];
+  unsigned long long hi = 0, lo = 0;
+  for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < c.n; i += (int64_t)gridDim.x * blockDim.x) {
+    if (is_null(col, i)) continue;
+    const unsigned long long k = ord_i64(ld_i64(col, i));
     hi = k > hi ? k : hi;
+    lo = ~k > lo ? ~k : lo;
   }
-  for (int o = 16; o > 0; o >>= 1) {
-    const long long l2 = __shfl_down_sync(WG_FULL_MASK, lo, o), h2 = __shfl_down_sync(WG_FULL_MASK, hi, o);
-    lo = l2 < lo ? l2 : lo;
-    hi = h2 > hi ? h2 : hi;
-  }
-  __shared__ long long s_lo[32], s_hi[32];
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31, nw = (blockDim.x + 31) >> 5;
-  if (l == 0) { s_lo[w] = lo; s_hi[w] = hi; }
-  __syncthreads();
-  if (w == 0) {
-    lo = l < nw ? s_lo[l] : LLONG_MAX;
-    hi = l < nw ? s_hi[l] : LLONG_MIN;
-    for (int o = 16; o > 0; o >>= 1) {
-      const long long l2 = __shfl_down_sync(WG_FULL_MASK, lo, o), h2 = __shfl_down_sync(WG_FULL_MASK, hi, o);
-      lo = l2 < lo ? l2 : lo;
-      hi = h2 > hi ? h2 : hi;
-    }
-    if (l == 0) {
-      atomicMin(mn, lo);
-      atomicMax(mx, hi);
-    }
+  hi = cta_reduce<true>(hi);
+  lo = cta_reduce<true>(lo);
+  if (threadIdx.x == 0) {
+    atomicMax(words + 2 * blockIdx.y, hi);
+    atomicMax(words + 2 * blockIdx.y + 1, lo);
   }
 }
 
@@ -262,8 +289,11 @@ __global__ void fill_u64_kernel(unsigned long long* out, int64_t n, unsigned lon
 }
 
 // Longest chain (max build rows sharing one key): the join's worst fan-out.
+// (2^21 slots, 2^19 chains of two: 345 us with an atomic per chain on the one
+// maximum, 9 us with one per CTA.)
 __global__ void join_fanout_kernel(JoinView j, unsigned long long* max_len) {
   const uint64_t cap = j.mask + 1;
+  unsigned long long most = 0;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < cap; i += (uint64_t)gridDim.x * blockDim.x) {
     int32_t head;
     if (j.flavor == 0) head = (int32_t)(((const unsigned long long*)j.slots)[i] >> 32);
@@ -271,8 +301,10 @@ __global__ void join_fanout_kernel(JoinView j, unsigned long long* max_len) {
     if (head < 0) continue;
     unsigned long long c = 0;
     for (int32_t r = head; r >= 0; r = j.next[r]) ++c;
-    atomicMax(max_len, c);
+    most = c > most ? c : most;
   }
+  most = cta_reduce<true>(most);
+  if (threadIdx.x == 0 && most) atomicMax(max_len, most);
 }
 
 __global__ void gather_kernel(const char* src, int64_t es, const uint64_t* valid, const int64_t* rows, int64_t n,
@@ -816,17 +848,26 @@ bool join_unique(wg_join* j) { return j->unique; }
 int32_t join_type_of(wg_join* j) { return j->jtype; }
 int64_t join_max_fanout(wg_join* j) { return j->max_fanout; }
 
+// The build's device scalars, one 64-bit word each: what the build kernels
+// find, read back together.
+enum : int { kSwDistinct = 0, kSwDup, kSwFanout, kSwRange, kSwWords = kSwRange + 2 * (1 + WG_MAX_PAYLOAD) };
+
+static wg_status clear_scalars(wg_join* j) {
+  WG_TRY(j->scratch.ensure(j->ctx, kSwWords * 8));
+  WG_CUDA_TRY(cudaMemsetAsync(j->scratch.get(), 0, kSwWords * 8, j->ctx->stream));
+  return WG_OK;
+}
+
 // The hash index (slots/next): one CAS insert per build row, heads chained
-// through `next`; counts distinct keys and flags duplicates.
-static wg_status build_hash(wg_join* j) {
+// through `next`; counts distinct keys and flags duplicates (hash_done takes
+// them from the scalars read back).
+static wg_status launch_hash(wg_join* j) {
   Ctx* ctx = j->ctx;
   const uint64_t cap = j->capacity;
   const int64_t slot_bytes = j->flavor == 0 ? 8 : 16;
   WG_TRY(j->slots.ensure(ctx, (int64_t)cap * slot_bytes));
   WG_TRY(j->next.ensure(ctx, std::max<int64_t>(j->rows, 1) * 4));
-  WG_TRY(j->scratch.ensure(ctx, 64));
   WG_CUDA_TRY(cudaMemsetAsync(j->slots.get(), 0xFF, (size_t)(cap * slot_bytes), ctx->stream));
-  WG_CUDA_TRY(cudaMemsetAsync(j->scratch.get(), 0, 64, ctx->stream));
   if (j->rows > 0) {
     BuildArgs a;
     a.key = wgd::DCol{j->key.data.get(), j->key.has_valid ? j->key.valid.as<uint64_t>() : nullptr,
@@ -837,20 +878,66 @@ static wg_status build_hash(wg_join* j) {
     a.mask = cap - 1;
     a.slots = j->slots.get();
     a.next = j->next.as<int32_t>();
-    a.distinct = j->scratch.as<unsigned long long>();
-    a.dup = (int32_t*)(j->scratch.as<char>() + 8);
+    a.distinct = j->scratch.as<unsigned long long>() + kSwDistinct;
+    a.dup = (int32_t*)(j->scratch.as<unsigned long long>() + kSwDup);
     a.err = ctx->dev_error;
     join_build_kernel<<<grid_for(ctx, j->rows, 256), 256, 0, ctx->stream>>>(a);
     ctx->count_launch();
     WG_CUDA_TRY(cudaGetLastError());
   }
-  int64_t back[2] = {0, 0};
-  WG_TRY(read_back_i64(ctx, j->scratch.as<int64_t>(), back, 2));
-  WG_TRY(check_device_error(ctx));
-  j->distinct = back[0];
-  j->unique = (int32_t)back[1] == 0;
-  j->hashed = true;
   return WG_OK;
+}
+
+static void hash_done(wg_join* j, const int64_t* scalars) {
+  j->distinct = scalars[kSwDistinct];
+  j->unique = (int32_t)scalars[kSwDup] == 0;
+  j->hashed = true;
+}
+
+static wg_status build_hash(wg_join* j) {
+  WG_TRY(clear_scalars(j));
+  WG_TRY(launch_hash(j));
+  int64_t back[kSwWords];
+  WG_TRY(read_back_checked(j->ctx, j->scratch.as<int64_t>(), back, kSwWords));
+  hash_done(j, back);
+  return WG_OK;
+}
+
+// Range words of the build key (column 0, when asked for) and of the integer
+// payload columns without NULLs; the others' words stay those of an empty range.
+static bool payload_ranged(const wg_join* j, size_t p) {
+  const int cls = class_of(j->pay[p].type_id);
+  return !j->pay[p].has_valid && (cls == WG_CLS_I32 || cls == WG_CLS_I64);
+}
+
+static wg_status launch_ranges(wg_join* j, bool with_key) {
+  Ctx* ctx = j->ctx;
+  RangeCols rc{};
+  rc.n = j->rows;
+  unsigned long long* words = j->scratch.as<unsigned long long>() + kSwRange;
+  for (size_t p = 0; p < 1 + j->pay.size() && j->rows > 0; ++p) {
+    // one launch per run of neighbouring columns that have a range (all of them, as a rule)
+    size_t q = p;
+    while (q < 1 + j->pay.size() && (q == 0 ? with_key : payload_ranged(j, q - 1))) {
+      const BuildCol& c = q == 0 ? j->key : j->pay[q - 1];
+      rc.col[q - p] = wgd::DCol{c.data.get(), c.has_valid ? c.valid.as<uint64_t>() : nullptr, class_of(c.type_id), 0};
+      ++q;
+    }
+    if (q == p) continue;
+    const dim3 grid(std::min<unsigned>(grid_for(ctx, j->rows, 256), (unsigned)ctx->sm_count * 8), (unsigned)(q - p));
+    range_kernel<<<grid, 256, 0, ctx->stream>>>(rc, words + 2 * p);
+    ctx->count_launch();
+    WG_CUDA_TRY(cudaGetLastError());
+    p = q;  // column q has no range
+  }
+  return WG_OK;
+}
+
+static long long range_lo(const int64_t* scalars, size_t col) {
+  return unord_i64(~(unsigned long long)scalars[kSwRange + 2 * col + 1]);
+}
+static long long range_hi(const int64_t* scalars, size_t col) {
+  return unord_i64((unsigned long long)scalars[kSwRange + 2 * col]);
 }
 
 // Unique int32 build keys without NULLs, spanning at most 4x the build rows,
@@ -871,43 +958,45 @@ static wg_status build_dense_unique(wg_join* j, bool* done) {
   if ((dsw && std::atoi(dsw) == 0) || (dns && std::atoi(dns) == 0) || j->rows <= 0 || j->flavor != 0 ||
       j->key.has_valid || j->pay.size() != 1 || j->pay[0].es != 4 || j->pay[0].has_valid)
     return WG_OK;
-  const int pcls = class_of(j->pay[0].type_id);
-  const bool pay_int = pcls == WG_CLS_I32 || pcls == WG_CLS_I64;
-  long long* mm = (long long*)(j->scratch.as<char>() + 16);  // key lo, hi, payload lo, hi
-  const long long init[4] = {LLONG_MAX, LLONG_MIN, LLONG_MAX, LLONG_MIN};
-  WG_CUDA_TRY(cudaMemcpyAsync(mm, init, 32, cudaMemcpyHostToDevice, ctx->stream));
-  wgd::DCol kd{j->key.data.get(), nullptr, class_of(j->key.type_id), 0};
-  key_range_kernel<<<grid_for(ctx, j->rows, 256), 256, 0, ctx->stream>>>(kd, j->rows, mm, mm + 1);
-  ctx->count_launch();
-  if (pay_int) {
-    wgd::DCol pd{j->pay[0].data.get(), nullptr, pcls, 0};
-    key_range_kernel<<<grid_for(ctx, j->rows, 256), 256, 0, ctx->stream>>>(pd, j->rows, mm + 2, mm + 3);
-    ctx->count_launch();
-  }
-  WG_CUDA_TRY(cudaGetLastError());
-  int64_t r[4];
-  WG_TRY(read_back_i64(ctx, (const int64_t*)mm, r, 4));
+  const bool pay_int = payload_ranged(j, 0);
+  WG_TRY(clear_scalars(j));
+  WG_TRY(launch_ranges(j, true));
+  int64_t back[kSwWords];
+  WG_TRY(read_back_i64(ctx, j->scratch.as<int64_t>(), back, kSwWords));
+  const long long klo = range_lo(back, 0), khi = range_hi(back, 0);
   int32_t sentinel;
-  if (r[0] > INT32_MIN) sentinel = (int32_t)(r[0] - 1);
-  else if (r[1] < INT32_MAX) sentinel = (int32_t)(r[1] + 1);
+  if (klo > INT32_MIN) sentinel = (int32_t)(klo - 1);
+  else if (khi < INT32_MAX) sentinel = (int32_t)(khi + 1);
   else return WG_OK;
-  const int64_t span = r[1] - r[0] + 1;
+  const int64_t span = khi - klo + 1;
   if (!(span > 0 && span <= std::max<int64_t>(4 * j->rows, 1024) && span <= (int64_t(1) << 30))) return WG_OK;
   const unsigned long long empty = (unsigned long long)(uint32_t)sentinel;
   WG_TRY(j->dslots.ensure(ctx, span * 8));
-  WG_CUDA_TRY(cudaMemsetAsync(j->scratch.get(), 0, 8, ctx->stream));
   fill_u64_kernel<<<grid_for(ctx, span, 256), 256, 0, ctx->stream>>>(j->dslots.as<unsigned long long>(), span, empty);
   ctx->count_launch();
+  wgd::DCol kd{j->key.data.get(), nullptr, class_of(j->key.type_id), 0};
   dense_build_kernel<<<grid_for(ctx, j->rows, 256), 256, 0, ctx->stream>>>(
-      kd, j->rows, j->pay[0].data.as<uint32_t>(), r[0], empty, j->dslots.as<unsigned long long>(),
-      j->scratch.as<int32_t>());
+      kd, j->rows, j->pay[0].data.as<uint32_t>(), klo, empty, j->dslots.as<unsigned long long>(),
+      (int32_t*)(j->scratch.as<unsigned long long>() + kSwDup));
   ctx->count_launch();
+  // unique keys fill their whole range: the payloads alone (half the bytes a
+  // probe's cache lines carry), queued before the duplicate flag is known
+  bool full = span == j->rows && env_full_dense();
+  if (full && j->dpay.ensure(ctx, span * 4) != WG_OK) {
+    full = false;  // no room for the copy: the dense table is probed as it is
+    set_error("");
+  }
+  if (full) {
+    dense_payload_kernel<<<grid_for(ctx, span, 256), 256, 0, ctx->stream>>>(j->dslots.as<unsigned long long>(), span,
+                                                                          j->dpay.as<uint32_t>());
+    ctx->count_launch();
+  }
   WG_CUDA_TRY(cudaGetLastError());
   int64_t dup = 0;
-  WG_TRY(read_back_i64(ctx, j->scratch.as<int64_t>(), &dup, 1));
+  WG_TRY(read_back_checked(ctx, j->scratch.as<int64_t>() + kSwDup, &dup, 1));
   if ((int32_t)dup != 0) return WG_OK;
-  j->pay_lo.assign(1, pay_int ? r[2] : 0);
-  j->pay_hi.assign(1, pay_int ? r[3] : 0);
+  j->pay_lo.assign(1, pay_int ? range_lo(back, 1) : 0);
+  j->pay_hi.assign(1, pay_int ? range_hi(back, 1) : 0);
   j->pay_range.assign(1, pay_int);
   j->distinct = j->rows;
   j->unique = true;
@@ -915,18 +1004,9 @@ static wg_status build_dense_unique(wg_join* j, bool* done) {
   j->direct = true;
   j->dense = true;
   j->sentinel = sentinel;
-  j->dense_base = r[0];
+  j->dense_base = klo;
   j->dense_slots = span;
-  // unique keys filling their whole range: the payloads alone (half the bytes a probe's cache lines carry)
-  j->full = false;
-  if (span == j->rows && env_full_dense()) {
-    WG_TRY(j->dpay.ensure(ctx, span * 4));
-    dense_payload_kernel<<<grid_for(ctx, span, 256), 256, 0, ctx->stream>>>(j->dslots.as<unsigned long long>(), span,
-                                                                          j->dpay.as<uint32_t>());
-    ctx->count_launch();
-    WG_CUDA_TRY(cudaGetLastError());
-    j->full = true;
-  }
+  j->full = full;
   *done = true;
   return WG_OK;
 }
@@ -996,45 +1076,43 @@ static wg_status build_finish_device(wg_join* j) {
   j->capacity = cap;
   j->shift = 64 - log2;
   j->hashed = false;
-  WG_TRY(j->scratch.ensure(ctx, 64));
   bool done = false;
   WG_TRY(build_dense_unique(j, &done));
   if (done) {
     j->finished = true;
-    return check_device_error(ctx);
+    return WG_OK;  // its read-back checked the device error word
   }
-  WG_TRY(build_hash(j));
+  // the hash index, the value ranges of the integer payload columns without
+  // NULLs, and the key's range where a direct table may follow: one wait
+  const char* dsw = std::getenv("WG_JOIN_DIRECT");
+  const bool direct_ok = (!dsw || std::atoi(dsw) != 0) && j->flavor == 0 && j->pay.size() == 1 && j->pay[0].es == 4 &&
+                         !j->pay[0].has_valid && j->rows > 0;
+  int64_t back[kSwWords];
+  WG_TRY(clear_scalars(j));
+  WG_TRY(launch_hash(j));
+  WG_TRY(launch_ranges(j, direct_ok));
+  WG_TRY(read_back_checked(ctx, j->scratch.as<int64_t>(), back, kSwWords));
+  hash_done(j, back);
   j->finished = true;
   j->max_fanout = 1;
   if (!j->unique) {
     wgd::JoinView v;
     WG_TRY(join_view(j, &v));
-    WG_CUDA_TRY(cudaMemsetAsync(j->scratch.get(), 0, 8, ctx->stream));
-    join_fanout_kernel<<<grid_for(ctx, (int64_t)cap, 256), 256, 0, ctx->stream>>>(v, j->scratch.as<unsigned long long>());
+    join_fanout_kernel<<<std::min<unsigned>(grid_for(ctx, (int64_t)cap, 256), (unsigned)ctx->sm_count * 8), 256, 0,
+                         ctx->stream>>>(v, j->scratch.as<unsigned long long>() + kSwFanout);
     ctx->count_launch();
     WG_CUDA_TRY(cudaGetLastError());
     int64_t mf = 1;
-    WG_TRY(read_back_i64(ctx, j->scratch.as<int64_t>(), &mf, 1));
+    WG_TRY(read_back_i64(ctx, j->scratch.as<int64_t>() + kSwFanout, &mf, 1));
     j->max_fanout = std::max<int64_t>(1, mf);
   }
-  // value range of the integer payload columns without NULLs
   j->pay_lo.assign(j->pay.size(), 0);
   j->pay_hi.assign(j->pay.size(), 0);
   j->pay_range.assign(j->pay.size(), false);
   for (size_t p = 0; p < j->pay.size() && j->rows > 0; ++p) {
-    const int cls = class_of(j->pay[p].type_id);
-    if (j->pay[p].has_valid || (cls != WG_CLS_I32 && cls != WG_CLS_I64)) continue;
-    long long* mm = (long long*)(j->scratch.as<char>() + 32);
-    const long long init[2] = {LLONG_MAX, LLONG_MIN};
-    WG_CUDA_TRY(cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, ctx->stream));
-    wgd::DCol pd{j->pay[p].data.get(), nullptr, cls, 0};
-    key_range_kernel<<<grid_for(ctx, j->rows, 256), 256, 0, ctx->stream>>>(pd, j->rows, mm, mm + 1);
-    ctx->count_launch();
-    WG_CUDA_TRY(cudaGetLastError());
-    int64_t r[2];
-    WG_TRY(read_back_i64(ctx, (const int64_t*)mm, r, 2));
-    j->pay_lo[p] = r[0];
-    j->pay_hi[p] = r[1];
+    if (!payload_ranged(j, p)) continue;
+    j->pay_lo[p] = range_lo(back, p + 1);
+    j->pay_hi[p] = range_hi(back, p + 1);
     j->pay_range[p] = true;
   }
   // Direct-payload table for the fused probe: unique int32 keys, exactly one
@@ -1042,18 +1120,9 @@ static wg_status build_finish_device(wg_join* j) {
   j->direct = false;
   j->dense = false;
   j->full = false;
-  const char* dsw = std::getenv("WG_JOIN_DIRECT");
-  if ((!dsw || std::atoi(dsw) != 0) && j->unique && j->flavor == 0 && j->pay.size() == 1 && j->pay[0].es == 4 &&
-      !j->pay[0].has_valid && j->rows > 0) {
-    long long* mm = (long long*)(j->scratch.as<char>() + 16);
-    const long long init[2] = {LLONG_MAX, LLONG_MIN};
-    WG_CUDA_TRY(cudaMemcpyAsync(mm, init, 16, cudaMemcpyHostToDevice, ctx->stream));
+  if (direct_ok && j->unique) {
+    const long long r[2] = {range_lo(back, 0), range_hi(back, 0)};
     wgd::DCol kd{j->key.data.get(), j->key.has_valid ? j->key.valid.as<uint64_t>() : nullptr, class_of(j->key.type_id), 0};
-    key_range_kernel<<<grid_for(ctx, j->rows, 256), 256, 0, ctx->stream>>>(kd, j->rows, mm, mm + 1);
-    ctx->count_launch();
-    WG_CUDA_TRY(cudaGetLastError());
-    int64_t r[2];
-    WG_TRY(read_back_i64(ctx, (const int64_t*)mm, r, 2));
     bool ok = true;
     if (r[0] > INT32_MIN) j->sentinel = (int32_t)(r[0] - 1);
     else if (r[1] < INT32_MAX) j->sentinel = (int32_t)(r[1] + 1);
