@@ -1,11 +1,18 @@
 // wg_filter.cu — exec.KernelFilter on the GPU (internal/engine/exec/filter.go:347-425).
 //
-// One pass over the column: each thread evaluates 4 × V rows with 128-bit
+// One pass over the column: each thread evaluates 8 × V rows with 128-bit
 // vector loads (V = 16 / element size), every row's verdict becomes a bit of a
 // warp ballot-style count, a block-wide scan orders the survivors, and the
 // tile's position in the output comes from a decoupled look-back over the
 // preceding tiles (Merrill & Garland, "Single-pass Parallel Prefix Scan with
-// Decoupled Look-back", NVIDIA TR 2016). Output is the ascending selection
+// Decoupled Look-back", NVIDIA TR 2016).
+//
+// What bounds it on long columns is the look-back, not memory: a tile's prefix
+// is known one status read (about 0.7 us) per window of predecessors after its
+// own count, so at most one window of tiles resolves per read latency. With a
+// 32-tile window that is 46 tiles of 8192 rows per microsecond: 2^28 int32 rows
+// took 656 us, 50 tiles per microsecond. Four status words per lane make it 128
+// tiles: 438 us, 80% of the rows kept. Output is the ascending selection
 // vector the reference's compaction produces, so the result is bit-exact.
 // Every wait on a predecessor tile is bounded; on expiry the kernel records
 // WG_DERR_TIMEOUT and publishes its own state so no successor waits forever.
@@ -59,6 +66,8 @@ using namespace wgd;
 
 constexpr int kBlock = 256;
 constexpr int kRows = 8;
+constexpr int kPerLane = 4;               // status words a lane of the look-back reads per step
+constexpr int kWindow = 32 * kPerLane;    // predecessors per step
 constexpr unsigned long long kFlagAgg = 1ULL << 62;
 constexpr unsigned long long kFlagInc = 2ULL << 62;
 constexpr unsigned long long kValMask = (1ULL << 62) - 1;
@@ -111,25 +120,45 @@ __global__ void __launch_bounds__(kBlock) filter_compact_kernel(const FilterArgs
   __shared__ uint32_t s_out[kTile];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  if (tid == 0) s_tile = atomicAdd(a.tile_counter, 1);
-  __syncthreads();
-  const int64_t tile = s_tile;
+  // tiles in the order the CTAs start, so a tile's predecessors are running or done
+  int64_t tile = 0;
+  if (a.num_tiles > 1) {
+    if (tid == 0) s_tile = atomicAdd(a.tile_counter, 1);
+    __syncthreads();
+    tile = s_tile;
+  }
   const int64_t tile_base = tile * kTile;
   const T cval = (CLS == WG_CLS_F32 || CLS == WG_CLS_F64) ? (T)a.p.cf : (T)a.p.ci;
 
   unsigned bits[kRows];
-  int excl[kRows];
+  if (VEC && tile_base + kTile <= a.n) {
+    // a whole tile: every load in flight before the first comparison
+    using W = typename VecOf<T>::type;
+    const W* src = reinterpret_cast<const W*>((const T*)a.col.data + tile_base) + tid;
+    W v[kRows];
 #pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const int64_t i0 = tile_base + ((int64_t)r * kBlock + tid) * V;
-    unsigned b = 0;
-    if (a.sel == nullptr && VEC && i0 + V <= a.n) {
-      typename VecOf<T>::type v = __ldg(reinterpret_cast<const typename VecOf<T>::type*>((const T*)a.col.data + i0));
-      const T* e = reinterpret_cast<const T*>(&v);
+    for (int r = 0; r < kRows; ++r) v[r] = __ldcs(src + r * kBlock);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const T* e = reinterpret_cast<const T*>(&v[r]);
+      unsigned b = 0;
 #pragma unroll
       for (int k = 0; k < V; ++k)
-        if (cmp_op<T>(e[k], cval, OP) && !is_null(a.col, i0 + k)) b |= 1u << k;
-    } else {
+        if (cmp_op<T>(e[k], cval, OP)) b |= 1u << k;
+      bits[r] = b;
+    }
+    if (a.col.valid != nullptr) {  // the first row is a multiple of V: V validity bits lie in one word
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) {
+        const int64_t i0 = tile_base + ((int64_t)r * kBlock + tid) * V;
+        bits[r] &= (unsigned)(__ldg(a.col.valid + (i0 >> 6)) >> (i0 & 63));
+      }
+    }
+  } else {
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int64_t i0 = tile_base + ((int64_t)r * kBlock + tid) * V;
+      unsigned b = 0;
 #pragma unroll
       for (int k = 0; k < V; ++k) {
         const int64_t it = i0 + k;
@@ -138,60 +167,101 @@ __global__ void __launch_bounds__(kBlock) filter_compact_kernel(const FilterArgs
           if (!is_null(a.col, row) && cmp_op<T>(__ldg((const T*)a.col.data + row), cval, OP)) b |= 1u << k;
         }
       }
+      bits[r] = b;
     }
-    bits[r] = b;
-    // warp inclusive scan of this thread's survivor count
-    int c = __popc(b), incl = c;
+  }
+  // warp scans of the survivor counts, four rows per word: a warp's count of one
+  // row is at most 32 * V <= 128, so bytes do not carry
+  static_assert(32 * V < 256 && kRows == 8, "packed counts");
+  unsigned own[2] = {0, 0}, incl4[2];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) own[r >> 2] |= (unsigned)__popc(bits[r]) << ((r & 3) * 8);
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    unsigned x = own[h];
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-      int y = __shfl_up_sync(WG_FULL_MASK, incl, d);
-      if (lane >= d) incl += y;
+      const unsigned y = __shfl_up_sync(WG_FULL_MASK, x, d);
+      if (lane >= d) x += y;
     }
-    excl[r] = incl - c;
+    incl4[h] = x;
+  }
+  int excl[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) {
+    const int incl = (int)(incl4[r >> 2] >> ((r & 3) * 8) & 255u);
+    excl[r] = incl - __popc(bits[r]);
     if (lane == 31) s_warp[r][warp] = incl;
   }
   __syncthreads();
-  // Decoupled look-back by warp 0: each step reads the status words of the 32
-  // closest unread predecessors at once, waits (bounded) until all of them
-  // have published, and adds their aggregates up to the closest inclusive one.
+  // Decoupled look-back by warp 0: each step reads the status words of the
+  // kWindow closest unread predecessors at once (four per lane), waits (bounded)
+  // until all of them have published, and adds their aggregates up to the
+  // closest inclusive one.
   if (warp == 0) {
-    int run = 0;
-    if (lane == 0) {
-      for (int r = 0; r < kRows; ++r)
-        for (int w = 0; w < kBlock / 32; ++w) { int t = s_warp[r][w]; s_warp[r][w] = run; run += t; }
-      s_total = run;
-      atomicExch(a.status + tile, (tile == 0 ? kFlagInc : kFlagAgg) | (unsigned long long)run);
+    // exclusive scan of the tile's kRows x warps counts, in row order
+    static_assert(kRows * (kBlock / 32) == 64, "two counts per lane");
+    int* cnt = &s_warp[0][0];
+    const int c0 = cnt[2 * lane], c1 = cnt[2 * lane + 1];
+    int incl = c0 + c1;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int y = __shfl_up_sync(WG_FULL_MASK, incl, d);
+      if (lane >= d) incl += y;
     }
-    run = __shfl_sync(WG_FULL_MASK, run, 0);
+    cnt[2 * lane] = incl - c0 - c1;
+    cnt[2 * lane + 1] = incl - c1;
+    const int run = __shfl_sync(WG_FULL_MASK, incl, 31);
+    if (lane == 0) {
+      s_total = run;
+      if (a.num_tiles > 1) atomicExch(a.status + tile, (tile == 0 ? kFlagInc : kFlagAgg) | (unsigned long long)run);
+    }
     long long prefix = 0;
     if (tile > 0) {
       int64_t tail = tile - 1;
       long long spins = 0;
       bool expired = false;
       for (;;) {
-        const int64_t idx = tail - lane;
-        unsigned long long st = idx >= 0 ? 0ULL : kFlagInc;  // before tile 0: an inclusive 0
+        const int64_t idx = tail - kPerLane * lane;  // this lane's predecessors: idx, idx - 1, ...
+        unsigned long long st[kPerLane];
+#pragma unroll
+        for (int q = 0; q < kPerLane; ++q) st[q] = idx - q >= 0 ? 0ULL : kFlagInc;  // before tile 0: an inclusive 0
         // the tile publishes its (partial) prefix on expiry, so no successor
         // waits forever and every position it writes stays below the true one
         for (;;) {
           if (spins >= a.spin_limit) { expired = true; break; }
-          if ((st & ~kValMask) == 0) st = *((volatile unsigned long long*)(a.status + idx));
-          if (!__any_sync(WG_FULL_MASK, (st & ~kValMask) == 0)) break;
+          bool missing = false;
+#pragma unroll
+          for (int q = 0; q < kPerLane; ++q) {
+            if ((st[q] & ~kValMask) == 0) st[q] = *((volatile unsigned long long*)(a.status + (idx - q)));
+          }
+#pragma unroll
+          for (int q = 0; q < kPerLane; ++q) missing |= (st[q] & ~kValMask) == 0;
+          if (!__any_sync(WG_FULL_MASK, missing)) break;
           ++spins;
-          __nanosleep(64);
+          __nanosleep(32);
         }
         if (expired) {
           if (lane == 0) set_error(a.err, WG_DERR_TIMEOUT);
           break;
         }
-        const unsigned inc = __ballot_sync(WG_FULL_MASK, (st & ~kValMask) == kFlagInc);
-        const int stop = inc ? __ffs(inc) - 1 : 31;  // lanes 0..stop count
-        long long v = lane <= stop ? (long long)(st & kValMask) : 0LL;
+        // words up to the closest inclusive one count: all of the lanes before
+        // the first lane that holds one, that lane's up to it
+        long long v = 0;
+        bool inc = false;
+#pragma unroll
+        for (int q = 0; q < kPerLane; ++q) {
+          if (!inc) v += (long long)(st[q] & kValMask);
+          inc |= (st[q] & ~kValMask) == kFlagInc;
+        }
+        const unsigned have = __ballot_sync(WG_FULL_MASK, inc);
+        const int stop = have ? __ffs(have) - 1 : 31;
+        if (lane > stop) v = 0;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(WG_FULL_MASK, v, o);
         prefix += v;
-        if (inc) break;
-        tail -= 32;
+        if (have) break;
+        tail -= kWindow;
       }
       if (lane == 0) atomicExch(a.status + tile, kFlagInc | (unsigned long long)(prefix + run));
     }
@@ -247,7 +317,7 @@ struct wg_filter {
   bool resolved = false;
   int32_t type_id = -1;
   wgd::Pred dp{};
-  wg::DevBuf status, counter, out_sel, out_n;
+  wg::DevBuf status, out_sel;
   wg::StagedBatch staged;
 };
 
@@ -255,7 +325,7 @@ namespace wg {
 
 // Run the compaction over a device-resident column; *n_out is left on the device.
 wg_status filter_launch(Ctx* ctx, const wgd::Pred& p, const wg_column& col, const uint32_t* sel, int64_t n_items,
-                        uint32_t* out, int64_t* n_out_dev, DevBuf& status, DevBuf& counter) {
+                        uint32_t* out, int64_t* n_out_dev, DevBuf& status) {
   const int cls = class_of(col.type_id);
   const int64_t es = elem_size(col.type_id);
   const bool vec = sel == nullptr && ((uintptr_t)col.data % 16 == 0);
@@ -267,18 +337,17 @@ wg_status filter_launch(Ctx* ctx, const wgd::Pred& p, const wg_column& col, cons
     return WG_OK;
   }
   if (tiles > (1LL << 31) - 1) return fail(WG_E_INVALID, "batch too large");
-  WG_TRY(status.ensure(ctx, tiles * 8));
-  WG_TRY(counter.ensure(ctx, 16));
-  WG_CUDA_TRY(cudaMemsetAsync(status.get(), 0, (size_t)(tiles * 8), ctx->stream));
-  WG_CUDA_TRY(cudaMemsetAsync(counter.get(), 0, sizeof(int), ctx->stream));
+  // the tile counter, then the tiles' status words; a single tile needs neither
+  WG_TRY(status.ensure(ctx, 16 + tiles * 8));
+  if (tiles > 1) WG_CUDA_TRY(cudaMemsetAsync(status.get(), 0, (size_t)(16 + tiles * 8), ctx->stream));
   FilterArgs a;
   a.col = wgd::DCol{col.data, col.valid_words, cls, col.scale};
   a.p = p;
   a.sel = sel;
   a.n = n_items;
   a.out = out;
-  a.status = status.as<unsigned long long>();
-  a.tile_counter = counter.as<int>();
+  a.status = status.as<unsigned long long>() + 2;
+  a.tile_counter = status.as<int>();
   a.out_n = n_out_dev;
   a.err = ctx->dev_error;
   a.num_tiles = tiles;
@@ -299,6 +368,27 @@ wg_status filter_launch(Ctx* ctx, const wgd::Pred& p, const wg_column& col, cons
 }  // namespace wg
 
 using namespace wg;
+
+// The compaction and its count on the host. The count lies behind the device
+// error word, so one copy and one wait bring both (a 2048-row batch spent two
+// copies and two waits after its 5 us kernel); the lock keeps another
+// thread's launch on this context from writing the count in between.
+static wg_status filter_count(wg_filter* f, const wg_column& col, const uint32_t* sel, int64_t n_items, uint32_t* out,
+                              int64_t* out_n) {
+  Ctx* ctx = f->ctx;
+  int32_t err = 0;
+  {
+    std::lock_guard<std::mutex> g(ctx->mu);
+    int64_t* count = (int64_t*)((char*)ctx->dev_error + kErrorCountOffset);
+    WG_TRY(filter_launch(ctx, f->dp, col, sel, n_items, out, count, f->status));
+    WG_CUDA_TRY(cudaMemcpyAsync(ctx->host_scalar, ctx->dev_error, kErrorCountOffset + 8, cudaMemcpyDeviceToHost,
+                                ctx->stream));
+    WG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
+    err = *(const int32_t*)ctx->host_scalar;
+    *out_n = *(const int64_t*)((const char*)ctx->host_scalar + kErrorCountOffset);
+  }
+  return device_error_status(ctx, err);
+}
 
 static wg_status filter_resolve(wg_filter* f, const wg_batch_desc* in) {
   if (!in) return fail(WG_E_INVALID, "batch is NULL");
@@ -335,11 +425,7 @@ wg_status wg_filter_execute_device(wg_filter* f, const wg_batch_desc* in, uint32
   WG_TRY(filter_resolve(f, in));
   Ctx* ctx = f->ctx;
   const int64_t n_items = in->sel ? in->sel_len : in->len;
-  WG_TRY(f->out_n.ensure(ctx, 16));
-  WG_TRY(filter_launch(ctx, f->dp, in->cols[f->pred.col], in->sel, n_items, out_sel_dev, f->out_n.as<int64_t>(),
-                       f->status, f->counter));
-  WG_TRY(read_back_i64(ctx, f->out_n.as<int64_t>(), out_n, 1));
-  return check_device_error(ctx);
+  return filter_count(f, in->cols[f->pred.col], in->sel, n_items, out_sel_dev, out_n);
 }
 
 wg_status wg_filter_execute(wg_filter* f, const wg_batch_desc* in, uint32_t* out_sel, int64_t* out_n) {
@@ -353,12 +439,7 @@ wg_status wg_filter_execute(wg_filter* f, const wg_batch_desc* in, uint32_t* out
   WG_TRY(stage_batch(ctx, &one, &f->staged));
   const int64_t n_items = in->sel ? in->sel_len : in->len;
   WG_TRY(f->out_sel.ensure(ctx, std::max<int64_t>(n_items * 4, 16)));
-  WG_TRY(f->out_n.ensure(ctx, 16));
-  wgd::Pred p = f->dp;
-  WG_TRY(filter_launch(ctx, p, f->staged.cols[0], f->staged.desc.sel, n_items, f->out_sel.as<uint32_t>(),
-                       f->out_n.as<int64_t>(), f->status, f->counter));
-  WG_TRY(read_back_i64(ctx, f->out_n.as<int64_t>(), out_n, 1));
-  WG_TRY(check_device_error(ctx));
+  WG_TRY(filter_count(f, f->staged.cols[0], f->staged.desc.sel, n_items, f->out_sel.as<uint32_t>(), out_n));
   if (*out_n > 0) {
     WG_CUDA_TRY(cudaMemcpyAsync(out_sel, f->out_sel.get(), (size_t)(*out_n * 4), cudaMemcpyDeviceToHost, ctx->stream));
     WG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));

@@ -74,6 +74,7 @@ class Ledger {
 };
 
 struct Ctx;
+constexpr int kErrorCountOffset = 16;
 
 // Device buffer charged to a context's ledger; freed and released on reset.
 class DevBuf {
@@ -123,7 +124,8 @@ struct Ctx {
   // small pinned/device scalars for read-backs
   int64_t* host_scalar = nullptr;   // pinned, 64 slots
   int64_t* dev_scalar = nullptr;    // device, 64 slots
-  // device-side error word written by bounded waits / invariants
+  // device-side error word written by bounded waits / invariants (256 bytes; a
+  // launch's result count may lie kErrorCountOffset behind it, read back with it)
   int32_t* dev_error = nullptr;
   std::mutex mu;                    // serialises scalar read-backs
   // host-input pipeline runs: two device windows and (for pageable sources) two
