@@ -176,3 +176,59 @@ def test_batch_upload_runs_like_host_input(ctx):
         g.close()
     b.close()
     assert ctx.ledger()["used"] <= used - n * 16
+
+
+@pytest.mark.parametrize("t,dtype", [(I32, np.int32), (DEC, DEC_DTYPE)])
+@pytest.mark.parametrize("nulls", [False, True])
+@pytest.mark.parametrize("bw", [1, 7, 12])
+@pytest.mark.parametrize("rows", [1, 503, 8192, 8193, 70_001])
+def test_run_shapes_and_slices(ctx, t, dtype, nulls, bw, rows):
+    """Streams cut into long stretches of equal bit-packed runs, stretches of equal repeated runs,
+    empty runs and runs with long headers, over pages at the edges of a slice of 8192 rows."""
+    import wadjet_b200 as wg
+    from wadjet_b200 import pages
+    rng = np.random.default_rng(rows * 31 + bw)
+    card = 1 << bw
+    dict_vals = dec_array(rng.integers(-10**12, 10**12, card)) if t == DEC else rng.permutation(card).astype(np.int32)
+    valid = rng.random(rows) >= 0.3 if nulls else None
+    idx, out = [], bytearray()
+    need = rows if valid is None else int(valid.sum())
+    vb = (bw + 7) // 8
+    while sum(map(len, idx)) < need:
+        kind = rng.integers(0, 5)
+        if kind == 0:  # equal bit-packed runs
+            g = int(rng.choice([1, 63, 64, 200]))
+            for _ in range(int(rng.integers(1, 70))):
+                v = rng.integers(0, card, g * 8)
+                out += pages._varint(g << 1 | 1) + pages._bitpack(v, bw)
+                idx.append(v)
+        elif kind == 1:  # equal repeated runs of short and long counts
+            n = int(rng.choice([1, 8, 63, 64, 5000]))
+            for _ in range(int(rng.integers(1, 70))):
+                v = int(rng.integers(0, card))
+                out += pages._varint(n << 1) + v.to_bytes(vb, "little")
+                idx.append(np.full(n, v))
+        elif kind == 2:
+            out += pages._varint(1)  # a bit-packed run of no groups
+        elif kind == 3:
+            out += pages._varint(0) + int(rng.integers(0, card)).to_bytes(vb, "little")
+        else:
+            v = rng.integers(0, card, 8)
+            out += pages._varint(3) + pages._bitpack(v, bw)
+            idx.append(v)
+    idx = np.concatenate(idx + [np.zeros(0, np.int64)])[:need]
+    levels = pages.encode_levels(valid) if nulls else None
+    phys = pages.physical(dict_vals, t)
+    ch = pages.Chunk(t, [pages.Page(rows, bytes([bw]) + bytes(out), pages.ENC_RLE_DICTIONARY, levels)],
+                     scale=2 if t == DEC else 0, dictionary=phys)
+    plain = pages.chunk(np.arange(rows, dtype=np.int64), I64, valid, page_rows=30_000)
+    b = wg.DeviceBatch.decode(ctx, [ch, plain])
+    got, ok = _device_values(wg, b, 0, dtype, rows)
+    keep = np.ones(rows, bool) if valid is None else valid
+    if nulls:
+        np.testing.assert_array_equal(ok, valid)
+    np.testing.assert_array_equal(got[keep].view(np.uint8), np.ascontiguousarray(dict_vals[idx]).view(np.uint8))
+    assert not got[~keep].view(np.uint8).any()
+    got, ok = _device_values(wg, b, 1, np.int64, rows)
+    np.testing.assert_array_equal(got, np.where(keep, np.arange(rows), 0))
+    b.close()

@@ -3,6 +3,7 @@
 #include "wg_device.cuh"
 
 #include <condition_variable>
+#include <functional>
 #include <cstdlib>
 #include <cstdio>
 #include <thread>
@@ -15,12 +16,9 @@ struct CopyPool {
   std::mutex mu;
   std::condition_variable cv_job, cv_done;
   std::vector<std::thread> threads;
-  // the current job: piece i of n copies [i * per, min(bytes, (i + 1) * per))
-  char* dst = nullptr;
-  const char* src = nullptr;
-  int64_t bytes = 0, per = 0;
+  // the current job: fn(0) .. fn(n - 1)
+  const std::function<void(int)>* fn = nullptr;
   int n = 0, next = 0, left = 0;
-  uint64_t gen = 0;
   std::mutex job_mu;  // one job at a time
   explicit CopyPool(int t) {
     for (int i = 0; i < t; ++i) threads.emplace_back([this] { run(); });
@@ -30,14 +28,24 @@ struct CopyPool {
     for (;;) {
       cv_job.wait(lk, [&] { return next < n; });
       const int i = next++;
-      char* d = dst;
-      const char* s = src;
-      const int64_t b0 = (int64_t)i * per, b1 = std::min(bytes, b0 + per);
+      const std::function<void(int)>* f = fn;
       lk.unlock();
-      if (b1 > b0) std::memcpy(d + b0, s + b0, (size_t)(b1 - b0));
+      (*f)(i);
       lk.lock();
       if (--left == 0) cv_done.notify_all();
     }
+  }
+  void each(int count, const std::function<void(int)>& f) {
+    std::lock_guard<std::mutex> job(job_mu);
+    std::unique_lock<std::mutex> lk(mu);
+    fn = &f;
+    next = 0;
+    left = count;
+    n = count;
+    cv_job.notify_all();
+    cv_done.wait(lk, [&] { return left == 0; });
+    n = 0;
+    next = 0;
   }
 };
 CopyPool* copy_pool() {
@@ -59,20 +67,128 @@ void parallel_copy(void* dst, const void* src, int64_t bytes) {
     return;
   }
   CopyPool* p = copy_pool();
-  std::lock_guard<std::mutex> job(p->job_mu);
-  std::unique_lock<std::mutex> lk(p->mu);
   const int t = (int)p->threads.size();
-  p->dst = (char*)dst;
-  p->src = (const char*)src;
-  p->bytes = bytes;
-  p->per = ((bytes + t - 1) / t + 4095) & ~int64_t(4095);
-  p->n = (int)((bytes + p->per - 1) / p->per);
-  p->next = 0;
-  p->left = p->n;
-  p->cv_job.notify_all();
-  p->cv_done.wait(lk, [&] { return p->left == 0; });
-  p->n = 0;
-  p->next = 0;
+  const int64_t per = ((bytes + t - 1) / t + 4095) & ~int64_t(4095);
+  p->each((int)((bytes + per - 1) / per), [&](int i) {
+    const int64_t b0 = (int64_t)i * per, b1 = std::min(bytes, b0 + per);
+    std::memcpy((char*)dst + b0, (const char*)src + b0, (size_t)(b1 - b0));
+  });
+}
+
+// ---- host pieces to the device ------------------------------------------------
+// Windows of the image are gathered into the context's two pinned slots by the
+// host threads while the DMA engine sends the window before: from pageable
+// memory the driver stages a copy itself at about 14 GB/s, after a pass of
+// ours over fresh pages to gather it.
+wg_status send_pieces(Ctx* ctx, const std::vector<HostPiece>& pieces, int64_t bytes, char* dst) {
+  constexpr int64_t kSlot = int64_t(4) << 20;
+  constexpr int64_t kGrain = int64_t(256) << 10;  // bytes one thread's share of a window starts at
+  if (bytes <= 0) return WG_OK;
+  std::lock_guard<std::mutex> stage_lock(ctx->stage_mu);
+  const int64_t slot = std::min(kSlot, (bytes + 255) & ~int64_t(255));
+  if (ctx->pinned_bytes < 2 * slot) {
+    if (ctx->pinned) cudaFreeHost(ctx->pinned);
+    ctx->pinned = nullptr;
+    ctx->pinned_bytes = 0;
+    WG_CUDA_TRY(cudaHostAlloc(&ctx->pinned, (size_t)(2 * slot), cudaHostAllocDefault));
+    ctx->pinned_bytes = 2 * slot;
+  }
+  wg_status st = WG_OK;
+  auto step = [&](int64_t w0, int s, bool wait) -> wg_status {
+    const int64_t w1 = std::min(bytes, w0 + slot);
+    char* pin = (char*)ctx->pinned + s * slot;
+    if (wait) WG_CUDA_TRY(cudaEventSynchronize(ctx->h2d_done[s]));  // the slot's last copy has left it
+    // part [a, b) of the window, from the pieces that overlap it (ordered by offset)
+    auto gather = [&](int64_t a, int64_t b) {
+      size_t lo = 0, hi = pieces.size();
+      while (lo < hi) {  // the first piece ending after a
+        const size_t mid = (lo + hi) / 2;
+        if (pieces[mid].off + pieces[mid].len > a) hi = mid; else lo = mid + 1;
+      }
+      for (size_t i = lo; i < pieces.size() && pieces[i].off < b; ++i) {
+        const int64_t x = std::max(a, pieces[i].off), y = std::min(b, pieces[i].off + pieces[i].len);
+        if (y > x) std::memcpy(pin + (x - w0), (const char*)pieces[i].src + (x - pieces[i].off), (size_t)(y - x));
+      }
+    };
+    const int64_t len = w1 - w0;
+    const int parts = (int)std::min<int64_t>((int64_t)copy_pool()->threads.size(), len / kGrain);
+    if (parts <= 1) {
+      gather(w0, w1);
+    } else {
+      const int64_t per = ((len + parts - 1) / parts + 63) & ~int64_t(63);
+      copy_pool()->each((int)((len + per - 1) / per), [&](int i) {
+        gather(w0 + i * per, std::min(w1, w0 + (i + 1) * per));
+      });
+    }
+    WG_CUDA_TRY(cudaMemcpyAsync(dst + w0, pin, (size_t)len, cudaMemcpyHostToDevice, ctx->stream));
+    WG_CUDA_TRY(cudaEventRecord(ctx->h2d_done[s], ctx->stream));
+    return WG_OK;
+  };
+  int64_t k = 0;
+  for (int64_t w0 = 0; w0 < bytes && st == WG_OK; w0 += slot, ++k) st = step(w0, (int)(k & 1), k >= 2);
+  // the slots belong to the next user of the lock
+  const cudaError_t e = cudaStreamSynchronize(ctx->stream);
+  if (st == WG_OK && e != cudaSuccess) return fail(WG_E_CUDA, std::string("staging: ") + cudaGetErrorString(e));
+  return st;
+}
+
+// ---- parked blocks ---------------------------------------------------------
+// Device blocks of finished decodes, for the next one: a cudaMalloc and a
+// cudaFree of tens of megabytes cost milliseconds each on a device that holds
+// other large allocations (40 of them 18 and 21 ms of a 2^21-row scan).
+// At most kParkBytes per context and a sixteenth of its budget; outside the
+// ledger while parked (in it again once taken); dropped when the device runs
+// out of memory and with the context.
+constexpr int64_t kParkBytes = int64_t(256) << 20;
+
+wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out) {
+  {
+    std::lock_guard<std::mutex> g(ctx->park_mu);
+    size_t best = ctx->parked.size();
+    for (size_t i = 0; i < ctx->parked.size(); ++i)
+      if (ctx->parked[i].bytes >= bytes && ctx->parked[i].bytes <= 2 * bytes + (int64_t(1) << 20) &&
+          (best == ctx->parked.size() || ctx->parked[i].bytes < ctx->parked[best].bytes))
+        best = i;
+    if (best < ctx->parked.size() && ctx->ledger.reserve(ctx->parked[best].bytes)) {
+      out->reset();
+      out->ctx_ = ctx;
+      out->ptr_ = ctx->parked[best].ptr;
+      out->bytes_ = ctx->parked[best].bytes;
+      ctx->parked.erase(ctx->parked.begin() + (int64_t)best);
+      return WG_OK;
+    }
+  }
+  return out->alloc(ctx, bytes);
+}
+
+void park_block(Ctx* ctx, DevBuf* b) {
+  if (!b->ptr_) return;
+  const int64_t most = std::min<int64_t>(kParkBytes, ctx->ledger.budget() > 0 ? ctx->ledger.budget() / 16 : kParkBytes);
+  std::lock_guard<std::mutex> g(ctx->park_mu);
+  int64_t held = b->bytes_;
+  for (const auto& p : ctx->parked) held += p.bytes;
+  while (held > most && !ctx->parked.empty()) {  // the oldest go first
+    held -= ctx->parked.front().bytes;
+    cudaFree(ctx->parked.front().ptr);
+    ctx->parked.erase(ctx->parked.begin());
+  }
+  if (held > most) {
+    b->reset();
+    return;
+  }
+  ctx->parked.push_back({b->ptr_, b->bytes_});
+  ctx->ledger.release(b->bytes_);
+  b->ctx_ = nullptr;
+  b->ptr_ = nullptr;
+  b->bytes_ = 0;
+}
+
+bool drop_parked(Ctx* ctx) {
+  std::lock_guard<std::mutex> g(ctx->park_mu);
+  const bool any = !ctx->parked.empty();
+  for (const auto& p : ctx->parked) cudaFree(p.ptr);
+  ctx->parked.clear();
+  return any;
 }
 
 thread_local std::string t_err;
@@ -100,6 +216,10 @@ wg_status DevBuf::alloc(Ctx* ctx, int64_t bytes) {
                                 ", budget=" + std::to_string(ctx->ledger.budget()) + ")");
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, (size_t)rounded);
+  if (e == cudaErrorMemoryAllocation && drop_parked(ctx)) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, (size_t)rounded);
+  }
   if (e != cudaSuccess) {
     ctx->ledger.release(rounded);
     cudaGetLastError();
@@ -295,6 +415,7 @@ wg_status wg_ctx_destroy(wg_ctx* c) {
     if (c->h2d_done[i]) cudaEventDestroy(c->h2d_done[i]);
     c->win[i].reset();
   }
+  drop_parked(c);
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->host_scalar) cudaFreeHost(c->host_scalar);
   if (c->dev_scalar) cudaFree(c->dev_scalar);

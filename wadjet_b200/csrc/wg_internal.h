@@ -100,6 +100,8 @@ class DevBuf {
   int64_t bytes() const { return bytes_; }
 
  private:
+  friend wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out);
+  friend void park_block(Ctx* ctx, DevBuf* b);
   Ctx* ctx_ = nullptr;
   void* ptr_ = nullptr;
   int64_t bytes_ = 0;
@@ -133,6 +135,13 @@ struct Ctx {
   std::mutex stage_mu;
   DevBuf win[2];
   cudaEvent_t h2d_done[2] = {nullptr, nullptr};
+  // device blocks kept for reuse (take_block / park_block)
+  struct Parked {
+    void* ptr;
+    int64_t bytes;
+  };
+  std::vector<Parked> parked;
+  std::mutex park_mu;
 
   explicit Ctx(int64_t budget, Ledger* parent = nullptr) : ledger(budget, parent) {}
   void count_launch(int n = 1) { launches.fetch_add(n); }
@@ -142,6 +151,23 @@ struct Ctx {
 // every context, sized to the host's cores): the pageable-to-pinned leg of
 // host-input staging.
 void parallel_copy(void* dst, const void* src, int64_t bytes);
+
+// A range of a device image that lies in host memory; `pieces` ordered by offset
+// and disjoint (bytes between them are left as they are or zero-filled at will).
+struct HostPiece {
+  const void* src;
+  int64_t off, len;
+};
+// The pieces to dst + off on the device, through pinned slots; the copies have
+// left host memory and reached the device on return.
+wg_status send_pieces(Ctx* ctx, const std::vector<HostPiece>& pieces, int64_t bytes, char* dst);
+
+// A device block of at least `bytes` for a buffer that the context's stream
+// alone uses, charged to the ledger: a parked one that fits, else a new one.
+// park_block gives it back once no queued work on any stream uses it.
+wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out);
+void park_block(Ctx* ctx, DevBuf* b);
+bool drop_parked(Ctx* ctx);
 
 wg_status ensure_device(Ctx* ctx);           // cudaSetDevice(ctx->device)
 wg_status read_back_i64(Ctx* ctx, const int64_t* dev, int64_t* out, int n);
