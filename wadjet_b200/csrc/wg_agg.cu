@@ -1134,6 +1134,7 @@ static wg_status run_device(const PipelineRun& r) {
     WG_TRY(agg_check_nullable(a, vs));
   }
   ls.P.err = ctx->dev_error;
+  ls.smem_half = (int64_t)ctx->max_smem_optin / 2 - 2048;
   const int64_t n_items = ls.P.n_items;
   if (n_items == 0) return WG_OK;
   const int64_t fan = r.join ? std::max<int64_t>(1, join_max_fanout(r.join)) : 1;

@@ -11,11 +11,10 @@ namespace wg {
 // The star-join shape's lean kernel (wg_star.cuh) when the launch is the
 // vector kernel with a shared table and the plan has its physical form
 // (WG_STAR_LEAN=0 keeps the generic vector kernel).
-template <int REP>
-static void launch_star_dense(const LaunchSpec& ls, cudaStream_t st) {
-  cudaFuncSetAttribute(wgd::starjoin_dense_kernel<REP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                       (int)ls.smem_bytes);
-  wgd::starjoin_dense_kernel<REP><<<ls.grid, 768, ls.smem_bytes, st>>>(ls.P);
+template <bool FIXED>
+static void launch_star_t(const LaunchSpec& l, cudaStream_t st) {
+  cudaFuncSetAttribute(wgd::starjoin_dense_kernel<FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem_bytes);
+  wgd::starjoin_dense_kernel<FIXED><<<l.grid, 768, l.smem_bytes, st>>>(l.P);
 }
 
 static bool launch_star_lean(const LaunchSpec& ls, cudaStream_t st) {
@@ -25,12 +24,18 @@ static bool launch_star_lean(const LaunchSpec& ls, cudaStream_t st) {
   }();
   if (!on || ls.vec == 0 || !ls.smem || ls.tile || ls.stage || ls.block != 768 || !wgd::starjoin_dense_ok(ls.P))
     return false;
-  switch (ls.P.smem_rep) {
-    case 1: launch_star_dense<1>(ls, st); return true;
-    case 2: launch_star_dense<2>(ls, st); return true;
-    case 4: launch_star_dense<4>(ls, st); return true;
-    default: launch_star_dense<8>(ls, st); return true;
-  }
+  // two words of fixed-point float SUM per slot while two CTAs still fit an SM
+  // (ls.smem_bytes holds for two: it was sized for at least one float copy)
+  LaunchSpec l = ls;
+  constexpr int sw = wgd::ShapeStarJoin::slot_words;
+  const int64_t fixed_bytes = (int64_t)l.P.smem_slots * ((sw + 2) | 1) * 8;
+  const bool fixed = fixed_bytes <= l.smem_half;
+  l.P.smem_rep = fixed ? -1 : 1;
+  l.P.smem_sw = fixed ? (sw + 2) | 1 : sw | 1;
+  l.smem_bytes = (size_t)l.P.smem_slots * l.P.smem_sw * 8;
+  if (fixed) launch_star_t<true>(l, st);
+  else launch_star_t<false>(l, st);
+  return true;
 }
 
 void launch_static_shape(const LaunchSpec& ls, cudaStream_t st) {

@@ -18,9 +18,14 @@
 // the probe drop the row; the DECIMAL operand is Int128.ToFloat64 then the
 // correctly rounded division by 10^scale (div_by_recip with the plan's divisor
 // pair); the projection is RN(price * RN(c1 - disc)) with c1 the program's
-// constant; a zero float contribution is skipped as apply() skips it; the
-// DECIMAL sum goes limb by limb; the row count is the slot's 32-bit counter;
-// float-SUM copies are lane-striped (copy lane % REP) and folded by the flush.
+// constant; the DECIMAL sum goes limb by limb; the row count is the slot's
+// 32-bit counter; the float SUM accumulates exactly, in fixed point at the
+// CTA's scale (f64_to_fixed_scaled), and is rounded once per CTA by the flush, so
+// its error is that of adding the CTAs' sums.
+//
+// What bounds it at 2^28 fact rows: 1939 us with the float SUM as four lane-striped float64
+// copies, 1546 without that SUM, 1482 without any table update, 1317 the copy
+// peak's time for its bytes; the two 32-bit limb adds bring it to 1688 us.
 #pragma once
 
 #include "wg_shapes.cuh"
@@ -30,24 +35,24 @@ namespace wgd {
 // Whether a plan (already matched to ShapeStarJoin, on the vector path with a
 // shared table) has the physical form the lean kernel serves.
 __host__ __forceinline__ bool starjoin_dense_ok(const Plan& P) {
-  return P.gdense && P.join.dense == 2 && P.smem_slots > 0 && P.smem_combine == 0 && P.sel == nullptr &&
-         (P.smem_rep == 1 || P.smem_rep == 2 || P.smem_rep == 4 || P.smem_rep == 8);
+  return P.gdense && P.join.dense == 2 && P.smem_slots > 0 && P.smem_combine == 0 && P.sel == nullptr;
 }
 
-template <int REP>
+// FIXED: the float SUM in two fixed-point words after the slot's; otherwise (a
+// table whose wider slots would leave room for one CTA per SM) one float64 word.
+template <bool FIXED>
 __global__ void __launch_bounds__(768, 2) starjoin_dense_kernel(const __grid_constant__ Plan P) {
   using C = ShapeStarJoin;
   static_assert(C::key_words == 1 && C::slot_words == 5 && C::agg_off(0) == 2 && C::agg_off(1) == 3,
                 "slot layout of the star-join shape");
   extern __shared__ unsigned long long sm[];
   __shared__ int s_groups;
+  __shared__ unsigned s_exp;
   Credit cr;
   const int S = P.smem_slots;
   smem_table_init(P, sm, S, &s_groups);
-  __syncthreads();
-  const int ssw = smem_stride(P);
+  const int ssw = smem_stride(P);  // the layout's words and two of the fixed-point float SUM, made odd
   const int lane = threadIdx.x & 31;
-  const int copy = lane & (REP - 1);  // this lane's float-SUM copy
   // columns: 0 qty int32, 1 fk int32, 2 price DECIMAL, 3 disc float64
   const int32_t* qty = (const int32_t*)P.in[0].data;
   const int32_t* fk = (const int32_t*)P.in[1].data;
@@ -64,6 +69,18 @@ __global__ void __launch_bounds__(768, 2) starjoin_dense_kernel(const __grid_con
   const int64_t n = P.n_items;
   const int64_t wpb = blockDim.x >> 5;
   const int64_t step = (int64_t)gridDim.x * wpb * 64;
+  // the float SUM's scale, from each thread's first row
+  double scale = 1.0;
+  if (FIXED) {
+    double first = 0.0;
+    const int64_t r = ((int64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * 64 + 2 * lane;
+    if (r < n) {
+      const longlong2 p0 = __ldg(price + r);
+      first = __dmul_rn(div_by_recip(int128_to_f64(p0.x, (unsigned long long)p0.y), db, dy), __dsub_rn(c1, __ldg(disc + r)));
+    }
+    scale = fixed_scale(fixed_exponent(first, &s_exp));
+  }
+  __syncthreads();  // the table is initialised
   for (int64_t base = ((int64_t)blockIdx.x * wpb + (threadIdx.x >> 5)) * 64; base < n; base += step) {
     const int64_t r0 = base + 2 * lane;
     int32_t q[2], f[2];
@@ -108,12 +125,14 @@ __global__ void __launch_bounds__(768, 2) starjoin_dense_kernel(const __grid_con
       const double pf = div_by_recip(int128_to_f64(ph[u], pl[u]), db, dy);
       const double v = __dmul_rn(pf, __dsub_rn(c1, d[u]));
       atomicAdd((unsigned*)(s + 1), 1u);
-      if (v != 0.0) atomicAdd((double*)(copy == 0 ? s + 2 : s + 5 + (copy - 1)), v);
+      unsigned long long flo, fhi;
+      if (FIXED && f64_to_fixed_scaled(v, scale, flo, fhi)) smem_add_limbs((unsigned*)(s + 5), 4, flo, fhi);
+      else if (v != 0.0) atomicAdd((double*)(s + 2), v);
       smem_add_limbs((unsigned*)(s + 3), 4, pl[u], (unsigned long long)ph[u]);
     }
   }
   __syncthreads();
-  smem_table_flush<2>(P, sm, S, cr);
+  smem_table_flush<2>(P, sm, S, cr, FIXED ? fixed_exponent_of(s_exp) : 64);
   cr.release(P.T);
 }
 
