@@ -1,0 +1,89 @@
+"""The row loop of compiled one-key group-by shapes (wg_lean.cuh) against the HBM-table path
+(WG_AGG_SMEM=0): keys of a small range (slot = key - base), sparse keys (hashed), a range with
+rows outside the sampled window, the key equal to the empty pattern, more groups than the hint
+gives room for, float SUM inputs of widely different magnitude (fixed point and its float
+fallback), and sizes around a lane's, a warp's and a CTA's rows.
+
+Integer state and MIN / MAX must be equal. Float sums: at most n additions of non-negative
+values in any order, so two orders differ by at most n * 2^-53 of the sum (below 1e-10 here);
+the infinite and NaN inputs must give the same infinities and NaNs."""
+import numpy as np
+import pytest
+
+from tests.helpers import canonical_order
+
+pytestmark = pytest.mark.gpu
+
+I32, I64, F64 = 1, 2, 4
+EMPTY = -0x7FFFFFFFFFFFFFFF
+
+
+def _keys(kind, n, rng):
+    if kind == "dense":
+        return rng.integers(-3000, 1000, n)
+    if kind == "sparse":
+        return rng.integers(0, 3000, n) * 0x1234567891
+    if kind == "outliers":  # nearly all keys in one range, a few far away on both sides
+        k = rng.integers(500, 900, n)
+        k[rng.random(n) < 0.002] = 1 << 62
+        k[rng.random(n) < 0.002] = -(1 << 62)
+        return k
+    if kind == "empty":
+        k = rng.integers(0, 50, n) + EMPTY - 10
+        return k
+    return rng.integers(0, 60_000, n)  # "many": more groups than the hint
+
+
+def _values(kind, n, rng):
+    if kind == "int":
+        return rng.integers(-(1 << 62), 1 << 62, n)
+    if kind == "wide":  # magnitudes over 2^-300 .. 2^300, zeros among them
+        return np.where(rng.random(n) < 0.1, 0.0, np.ldexp(rng.random(n), rng.integers(-300, 300, n)))
+    v = rng.random(n) * 1e5
+    if kind == "special":
+        v[rng.random(n) < 0.001] = np.inf
+        v[rng.random(n) < 0.0005] = np.nan
+    return v
+
+
+def _run(ctx, wg, shape, cols, hint, n):
+    key, val, filt = cols
+    if shape == "groupby":  # flag, k, v, f
+        a = wg.HashAggregate(ctx, [0], [wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1),
+                                        wg.AggColumn(wg.AGG_MIN, 3), wg.AggColumn(wg.AGG_MAX, 3)], ndv_hint=hint)
+        batch = wg.Batch([wg.Column(I64, key), wg.Column(I64, np.arange(n)), wg.Column(I32, filt), wg.Column(F64, val)])
+    else:
+        a = wg.HashAggregate(ctx, [0], [wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1),
+                                        wg.AggColumn(wg.AGG_MIN, 1), wg.AggColumn(wg.AGG_MAX, 1)], ndv_hint=hint)
+        batch = wg.Batch([wg.Column(I64, key), wg.Column(I64 if shape == "i64" else F64, val), wg.Column(I32, filt)])
+    wg.run_pipeline(ctx, batch, a, filters=[(2, wg.OP_LT, 7)])
+    a.finalize()
+    assert a.kernel_shape == {"groupby": 2, "i64": 4, "f64": 5}[shape]
+    e = a.export()
+    a.close()
+    return e
+
+
+@pytest.mark.parametrize("shape,values", [("groupby", "float"), ("i64", "int"), ("f64", "float"), ("f64", "wide"),
+                                          ("f64", "special")])
+@pytest.mark.parametrize("keys", ["dense", "sparse", "outliers", "empty", "many"])
+@pytest.mark.parametrize("n", [1, 127, 129, 4097, 100_003])
+def test_lean_equals_the_hbm_table(ctx, monkeypatch, shape, values, keys, n):
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(n + len(keys) * 7 + len(values))
+    cols = (_keys(keys, n, rng).astype(np.int64), _values(values, n, rng), rng.integers(0, 10, n, dtype=np.int32))
+    hint = 2000 if keys == "many" else 4000
+    monkeypatch.setenv("WG_AGG_SMEM", "1")
+    got = _run(ctx, wg, shape, cols, hint, n)
+    monkeypatch.setenv("WG_AGG_SMEM", "0")
+    want = _run(ctx, wg, shape, cols, hint, n)
+    og, ow = canonical_order(got), canonical_order(want)
+    for f in ("keys", "count", "i64", "has"):
+        np.testing.assert_array_equal(got[f][:, og], want[f][:, ow])
+    g, w = got["f64"][:, og], want["f64"][:, ow]
+    np.testing.assert_array_equal(g[2:], w[2:])  # MIN, MAX
+    if shape == "f64":
+        np.testing.assert_array_equal(np.isnan(g[0]), np.isnan(w[0]))
+        np.testing.assert_array_equal(np.isinf(g[0]), np.isinf(w[0]))
+        fin = np.isfinite(w[0])
+        assert (np.abs(g[0][fin] - w[0][fin]) <= 1e-10 * np.abs(w[0][fin])).all()

@@ -1067,6 +1067,20 @@ static int str_key_col(const wg_agg* a, const wg_batch_desc* in) {
   return kc >= 0 && kc < in->ncols && is_str_type(in->cols[kc].type_id) ? kc : -1;
 }
 
+// Rows of a CTA with a shared table: every CTA flushes up to all of the groups
+// into the HBM table at the end, all onto the same slots, so a small input takes
+// fewer CTAs. With r rows per CTA a launch takes about r * a + (n / r) * groups * b,
+// least at r = sqrt(n * groups * b / a); measured over 2^16..2^20 rows and
+// 16..4096 groups (r of 2048, 4096, 8192, 16384) the best r is a quarter of
+// sqrt(n * groups), not below 4096: 2^20 rows 17 / 19 / 31 / 62 us for 16 / 256 /
+// 1024 / 4096 groups, against 23 / 26 / 36 / 64 us with max(16384, 4 rows per slot);
+// 2^16 rows 12 / 14 / 21 / 31 against 21 / 24 / 30 / 46 us. WG_SMEM_ROWS_PER_CTA sets it.
+static int64_t smem_rows_per_cta(int64_t n, int64_t groups) {
+  const int64_t env = env_int("WG_SMEM_ROWS_PER_CTA", 0);
+  if (env > 0) return env;
+  return std::max<int64_t>(4096, (int64_t)(std::sqrt((double)n * (double)std::max<int64_t>(groups, 1)) / 4));
+}
+
 // Shared-memory launch of a plan without a compiled shape (lowcard_kernel), or
 // none (ls.smem false: the rows update the HBM table): the expected groups (or
 // the keys of a known range [glo, ghi]) must fit the key table at most 3/4
@@ -1102,8 +1116,7 @@ static void lowcard_setup(wg_agg* a, LaunchSpec& ls, int64_t expect, bool ranged
     ls.P.gmin = glo;
     ls.smem_bytes = (size_t)(S * key_bytes + R * (S + 2) * aw * 8);
     ls.block = lowcard_threads(ctas);
-    // a CTA flushes up to every slot into the HBM table: at least four rows per slot
-    const int64_t rows = std::max<int64_t>(std::max<int64_t>(lowcard_rows(ls.block), 4096), 4 * S);
+    const int64_t rows = std::max<int64_t>(lowcard_rows(ls.block), smem_rows_per_cta(ls.P.n_items, dense ? S : std::max<int64_t>(expect, 1)));
     ls.grid = (unsigned)std::min<int64_t>((int64_t)ctx->sm_count * ctas, (ls.P.n_items + rows - 1) / rows);
     return;
   }
@@ -1135,6 +1148,7 @@ static wg_status run_device(const PipelineRun& r) {
   }
   ls.P.err = ctx->dev_error;
   ls.smem_half = (int64_t)ctx->max_smem_optin / 2 - 2048;
+  ls.smem_whole = (int64_t)ctx->max_smem_optin - 2048;
   const int64_t n_items = ls.P.n_items;
   if (n_items == 0) return WG_OK;
   const int64_t fan = r.join ? std::max<int64_t>(1, join_max_fanout(r.join)) : 1;
@@ -1294,16 +1308,7 @@ static wg_status run_device(const PipelineRun& r) {
   const int mm = env_int("WG_MINMAX_TEST", -1);
   ls.P.minmax_test = mm >= 0 ? (mm != 0) : (n_items >= 8 * std::max<int64_t>(expect, 1));
   int64_t rows_per_cta = (int64_t)ls.block * (ls.vec ? ls.vec : 1);
-  // a CTA with a shared table flushes up to all of its slots into the HBM table
-  // at the end, every CTA onto the same hot groups: a small input takes fewer
-  // CTAs, each with at least four rows per slot (16K rows at least), so the
-  // flushes do not outweigh the rows (a 2^20-row query over 4096 groups: 80 us
-  // on 148 CTAs, all flushing every group)
-  if (ls.smem) {
-    const int64_t floor_rows = env_int("WG_SMEM_ROWS_PER_CTA", 0) > 0 ? env_int("WG_SMEM_ROWS_PER_CTA", 0)
-                                                                       : std::max<int64_t>(16384, 4 * (int64_t)S);
-    rows_per_cta = std::max(rows_per_cta, floor_rows);
-  }
+  if (ls.smem) rows_per_cta = std::max(rows_per_cta, smem_rows_per_cta(n_items, ls.P.gdense ? S : expect));
   const int64_t want_ctas = (n_items + rows_per_cta - 1) / rows_per_cta + 1;
   ls.grid = (unsigned)std::min<int64_t>((int64_t)ctx->sm_count * blocks_per_sm, want_ctas);
   if (!ls.smem && !stat) ls.grid = (unsigned)std::min<int64_t>((int64_t)ctx->sm_count * 4, (n_items + 1023) / 1024 + 1);

@@ -960,10 +960,11 @@ __device__ __forceinline__ void smem_table_init(const Plan& P, unsigned long lon
   fill_pattern(sm, (int64_t)S * ssw, ssw, sw, s_init, (int64_t)threadIdx.x, (int64_t)blockDim.x);
 }
 
-// fixed_exp: the exponent of the fixed-point float SUMs' scale (rep < 0).
+// fixed_exp: the exponent of the fixed-point float SUMs' scale (rep < 0);
+// dense, gmin: whether slot i holds key gmin + i, as the plan has it or a CTA chose.
 template <int NA>
 __device__ __forceinline__ void smem_table_flush(const Plan& P, const unsigned long long* sm, int S, Credit& cr,
-                                                 int fixed_exp = 64) {
+                                                 int fixed_exp, bool dense, long long gmin) {
   const LayoutAcc ly{P.L};
   const int sw = P.L.slot_words, ssw = smem_stride(P), rep = smem_copies(P);
   // CTAs start their pass at different slots: CTAs that finish together then
@@ -974,9 +975,9 @@ __device__ __forceinline__ void smem_table_flush(const Plan& P, const unsigned l
     const int i = i0 + off < S ? i0 + off : i0 + off - S;
     const unsigned long long* s = sm + (size_t)i * ssw;
     unsigned long long key = s[0];
-    if (P.gdense) {  // a direct slot is in use once it counted a row
+    if (dense) {  // a direct slot is in use once it counted a row
       if (s[P.L.key_words] == 0) continue;
-      key = (unsigned long long)P.gmin + (unsigned long long)i;
+      key = (unsigned long long)gmin + (unsigned long long)i;
     } else if (key == WG_EMPTY_KEY) {
       continue;
     }
@@ -996,6 +997,12 @@ __device__ __forceinline__ void smem_table_flush(const Plan& P, const unsigned l
     }
     apply<NA, false>(ly, g, c, s[P.L.key_words]);
   }
+}
+
+template <int NA>
+__device__ __forceinline__ void smem_table_flush(const Plan& P, const unsigned long long* sm, int S, Credit& cr,
+                                                 int fixed_exp = 64) {
+  smem_table_flush<NA>(P, sm, S, cr, fixed_exp, P.gdense != 0, P.gmin);
 }
 
 // One lane's share of the L2 prefetch of a grid-stride loop over chunks of

@@ -3,6 +3,7 @@
 #include "wg_internal.h"
 #include "wg_launch.cuh"
 #include "wg_star.cuh"
+#include "wg_lean.cuh"
 
 #include <cstdlib>
 
@@ -38,6 +39,32 @@ static bool launch_star_lean(const LaunchSpec& ls, cudaStream_t st) {
   return true;
 }
 
+// Shapes that group by one hashed integer key, on the vector path with a shared
+// table: lean_group_kernel, one CTA of 1024 threads per SM or two of 512.
+template <class C, bool FIXED>
+static void launch_lean_t(const LaunchSpec& l, unsigned block, cudaStream_t st) {
+  cudaFuncSetAttribute(wgd::lean_group_kernel<C, FIXED>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)l.smem_bytes);
+  wgd::lean_group_kernel<C, FIXED><<<l.grid, block, l.smem_bytes, st>>>(l.P);
+}
+
+template <class C>
+static bool launch_lean(const LaunchSpec& ls, cudaStream_t st) {
+  if (ls.vec == 0 || !ls.smem || ls.tile || ls.stage || ls.P.gdense || ls.P.smem_combine) return false;
+  LaunchSpec l = ls;
+  const bool whole = ls.block == 1024;  // the table takes a whole SM
+  constexpr bool any_float = wgd::lean_float_sums<C>() > 0;
+  // fixed-point float SUMs widen the slots: taken while the table keeps its CTAs per SM
+  const int64_t room = whole ? ls.smem_whole : ls.smem_half;
+  const bool fixed = any_float && (int64_t)l.P.smem_slots * wgd::lean_stride<C>(true) * 8 <= room;
+  l.P.smem_rep = fixed ? -1 : 1;
+  l.P.smem_sw = wgd::lean_stride<C>(fixed);
+  l.smem_bytes = (size_t)l.P.smem_slots * l.P.smem_sw * 8;
+  const unsigned block = whole ? wgd::kLeanThreads : wgd::kLeanThreads / 2;
+  if (fixed) launch_lean_t<C, any_float>(l, block, st);
+  else launch_lean_t<C, false>(l, block, st);
+  return true;
+}
+
 void launch_static_shape(const LaunchSpec& ls, cudaStream_t st) {
   using namespace wgd;
   switch (ls.P.shape) {
@@ -45,11 +72,23 @@ void launch_static_shape(const LaunchSpec& ls, cudaStream_t st) {
       if (launch_star_lean(ls, st)) return;
       launch_pipeline_t<ShapeStarJoin::n_aggs, StatShape<ShapeStarJoin>>(ls, st);
       return;
-    case SHAPE_GROUPBY: launch_pipeline_t<ShapeGroupBy::n_aggs, StatShape<ShapeGroupBy>>(ls, st); return;
+    case SHAPE_GROUPBY:
+      if (launch_lean<ShapeGroupBy>(ls, st)) return;
+      launch_pipeline_t<ShapeGroupBy::n_aggs, StatShape<ShapeGroupBy>>(ls, st);
+      return;
     case SHAPE_HIGHCARD: launch_pipeline_t<ShapeHighCard::n_aggs, StatShape<ShapeHighCard>>(ls, st); return;
-    case SHAPE_BATCH_I64: launch_pipeline_t<ShapeBatchI64::n_aggs, StatShape<ShapeBatchI64>>(ls, st); return;
-    case SHAPE_BATCH_F64: launch_pipeline_t<ShapeBatchF64::n_aggs, StatShape<ShapeBatchF64>>(ls, st); return;
-    case SHAPE_IPV4: launch_pipeline_t<ShapeIPv4::n_aggs, StatShape<ShapeIPv4>>(ls, st); return;
+    case SHAPE_BATCH_I64:
+      if (launch_lean<ShapeBatchI64>(ls, st)) return;
+      launch_pipeline_t<ShapeBatchI64::n_aggs, StatShape<ShapeBatchI64>>(ls, st);
+      return;
+    case SHAPE_BATCH_F64:
+      if (launch_lean<ShapeBatchF64>(ls, st)) return;
+      launch_pipeline_t<ShapeBatchF64::n_aggs, StatShape<ShapeBatchF64>>(ls, st);
+      return;
+    case SHAPE_IPV4:
+      if (launch_lean<ShapeIPv4>(ls, st)) return;
+      launch_pipeline_t<ShapeIPv4::n_aggs, StatShape<ShapeIPv4>>(ls, st);
+      return;
     default: return;
   }
 }

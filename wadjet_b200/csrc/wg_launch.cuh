@@ -19,7 +19,7 @@ struct LaunchSpec {
   int block = kAggBlock;
   unsigned grid = 1;
   size_t smem_bytes = 0;
-  int64_t smem_half = 0;      // shared memory each of two CTAs per SM may take
+  int64_t smem_half = 0, smem_whole = 0;  // shared memory each of two CTAs per SM may take, or one
   bool tile = false;          // TMA-staged tile kernel
   wgd::TileCfg cfg{};
   int vec = 0;                // compiled shapes: rows per lane of the vector kernel (0 = one-row kernel)

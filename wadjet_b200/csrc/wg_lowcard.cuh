@@ -345,7 +345,7 @@ __device__ __forceinline__ int lc_slot(const Plan& P, unsigned long long* keys, 
 // One row whose key found no shared slot, into the HBM table (rare: a hint far
 // below the groups there are). Neither inlined nor handed the key: it would hold
 // registers through every row's common path.
-__device__ __noinline__ void lc_far_row(const Plan& P, int64_t row, int32_t brow, Credit* cr) {
+static __device__ __noinline__ void lc_far_row(const Plan& P, int64_t row, int32_t brow, Credit* cr) {
   const DynShape sh{P};
   const SrcGlobal src{row};
   ExprVals ev;
