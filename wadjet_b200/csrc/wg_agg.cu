@@ -44,6 +44,12 @@ namespace {
 
 constexpr int64_t kSnapshotMaxBytes = 256LL << 20;
 constexpr double kMaxLoad = 0.75;
+// key windows (wg_window.cuh): inputs from this many rows on (five launches
+// instead of one, about 15 us more), slots of at most kWindowBytes in all and
+// eight per expected group
+constexpr int64_t kWindowMinRows = int64_t(1) << 20;
+constexpr int64_t kWindowBytes = int64_t(32) << 20;
+constexpr int64_t kWindowHeader = 256;
 // spill partitions take hash bits [20, 30): below the slot bits of any table up
 // to 2^34 slots, so each partition's keys spread over its whole table
 constexpr int kSpillPartShift = 20;
@@ -552,6 +558,8 @@ struct wg_agg {
   // the next query: allocating and freeing GBs per query costs milliseconds)
   std::vector<wg::DevBuf> part_bufs;
   wg::DevBuf part_counts, part_offs;
+  // a key window (its bounds, then its slots from kWindowHeader bytes on), kept for the next launch
+  wg::DevBuf win_buf;
   char* exp_host = nullptr;
   int64_t exp_host_bytes = 0;
   cudaEvent_t exp_ev[2] = {nullptr, nullptr};
@@ -896,6 +904,20 @@ static wg_status launch_pipeline(wg_agg* a, const LaunchSpec& ls, int64_t n_item
   if (l2.tile) l2.cfg.n_tiles = (n_items + l2.cfg.rows - 1) / l2.cfg.rows;
   P.shape = pick_shape(P);
   a->last_shape = P.shape;
+  P.win = nullptr;
+  if (l2.win && n_items >= kWindowMinRows) {
+    // both the window kernel and the table kernel are queued; the sampled
+    // window decides on the device which of them takes the rows
+    P.win = a->win_buf.as<wgd::KeyWindow>();
+    P.wslots = a->win_buf.as<unsigned long long>() + kWindowHeader / 8;
+    launch_window_begin(l2, ctx->sm_count, ctx->stream);
+    if (!launch_window_static(l2, ctx->sm_count, ctx->stream)) launch_window_rows(l2, ctx->sm_count, ctx->stream);
+    if (!l2.win_known) launch_pipeline_shape(l2, ctx->stream);
+    launch_window_fold(l2, ctx->sm_count, ctx->stream);
+    ctx->count_launch(l2.win_known ? 4 : 5);
+    WG_CUDA_TRY(cudaGetLastError());
+    return WG_OK;
+  }
   launch_pipeline_shape(l2, ctx->stream);
   ctx->count_launch();
   WG_CUDA_TRY(cudaGetLastError());
@@ -1373,6 +1395,26 @@ static wg_status run_device(const PipelineRun& r) {
     ls.lc = false;
     ls.P.smem_slots = 0;
     ls.smem_bytes = 0;
+  }
+  // Groups beyond shared memory keyed by one integer: a key window, its range
+  // known (an inner join's payload column, a dictionary's ids) or sampled
+  const int32_t shape = stat ? pick_shape(probe) : wgd::SHAPE_GENERIC;
+  const bool has_window = !stat || (ls.vec && shape != wgd::SHAPE_STARJOIN && shape != wgd::SHAPE_HIGHCARD);
+  if (has_window && !ls.smem && !ls.tile && a->L.key_words == 1 && a->L.n_keys == 1 && !a->spill &&
+      n_items >= kWindowMinRows && env_int("WG_KEY_WINDOW", 1) != 0) {
+    const int64_t slot = (int64_t)a->L.slot_words * 8;
+    const bool known = ranged && ghi >= glo && (uint64_t)ghi - (uint64_t)glo < (uint64_t)(kWindowBytes / slot);
+    int64_t slots = 0;
+    if (known) slots = ghi - glo + 1;
+    else if (!r.join && expect > 0) slots = std::min<int64_t>(8 * std::max<int64_t>(expect, 1024), kWindowBytes / slot);
+    if (slots > 0 && a->win_buf.ensure(ctx, kWindowHeader + slots * slot) == WG_OK) {
+      ls.win = true;
+      ls.win_known = known;
+      ls.win_base = known ? glo : 0;
+      ls.win_slots = slots;
+    } else if (slots > 0) {
+      set_error("");  // no room for the window: the table as it is
+    }
   }
   const wgd::Plan base = ls.P;
   // the room the launch policy plans with: the table's limit less the
@@ -2497,12 +2539,13 @@ Ctx* agg_ctx(wg_agg* a) { return a->ctx; }
 // Frees what an aggregate keeps only to speed up its next query (the
 // reordered input copy and its counters), for an aggregate parked in a pool.
 void agg_trim(wg_agg* a) {
-  if (a->part_bufs.empty() && !a->part_counts.get()) return;
+  if (a->part_bufs.empty() && !a->part_counts.get() && !a->win_buf.get()) return;
   ensure_device(a->ctx);
   cudaStreamSynchronize(a->ctx->stream);  // no launch still reads them
   a->part_bufs.clear();
   a->part_counts.reset();
   a->part_offs.reset();
+  a->win_buf.reset();
 }
 std::vector<int32_t> agg_input_cols(wg_agg* a) {
   std::vector<int32_t> r = a->key_cols;

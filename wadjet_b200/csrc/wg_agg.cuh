@@ -83,6 +83,12 @@ struct ExprD {
   long long imm[WG_EXPR_OPS];    // int immediate, or the bits of a float immediate
 };
 
+// Keys [base, base + n) whose groups a launch keeps in an array (wg_window.cuh); n = 0: none.
+struct KeyWindow {
+  long long base;
+  unsigned long long n;
+};
+
 struct Plan {
   int64_t n_items;
   const uint32_t* sel;           // nullptr = rows [0, n_items)
@@ -118,6 +124,8 @@ struct Plan {
   double vdiv_y[WG_MAX_IN + WG_MAX_PAYLOAD + WG_MAX_EXPRS];
   Layout L;
   Table T;
+  const KeyWindow* win;          // nullptr: no window; else set on the device before the launch's kernels
+  unsigned long long* wslots;    // the window's slots (L.slot_words words each, key words unused)
   int32_t* err;
 };
 

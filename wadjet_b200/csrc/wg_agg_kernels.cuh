@@ -1042,6 +1042,7 @@ template <int NA, bool SMEM, class Sh>
 __global__ void __launch_bounds__(Sh::kBlock, Sh::kMinBlocks) pipeline_kernel(const __grid_constant__ Plan P) {
   extern __shared__ unsigned long long sm[];
   __shared__ int s_groups;
+  if (!SMEM && P.win != nullptr && P.win->n != 0) return;  // the window kernel takes the rows
   const Sh sh{P};
   Credit cr;  // this thread's group reservations, handed back at the end
   const int S = P.smem_slots;
@@ -1457,6 +1458,7 @@ __global__ void __launch_bounds__(BLK, MB) pipeline_vec_kernel(const __grid_cons
   static_assert(U == 2 || U == 4, "rows per lane");
   extern __shared__ unsigned long long sm[];
   __shared__ int s_groups;
+  if (!SMEM && P.win != nullptr && P.win->n != 0) return;  // the window kernel takes the rows
   const Sh sh{P};
   Credit cr;  // this thread's group reservations, handed back at the end
   const int S = P.smem_slots;

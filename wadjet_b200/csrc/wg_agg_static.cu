@@ -4,7 +4,9 @@
 #include "wg_launch.cuh"
 #include "wg_star.cuh"
 #include "wg_lean.cuh"
+#include "wg_window.cuh"
 
+#include <algorithm>
 #include <cstdlib>
 
 namespace wg {
@@ -63,6 +65,26 @@ static bool launch_lean(const LaunchSpec& ls, cudaStream_t st) {
   if (fixed) launch_lean_t<C, any_float>(l, block, st);
   else launch_lean_t<C, false>(l, block, st);
   return true;
+}
+
+template <class C>
+static bool launch_window_t(const LaunchSpec& ls, int sms, cudaStream_t st) {
+  const int64_t per = (int64_t)wgd::kWinBlock * wgd::kWinRows;
+  const unsigned grid = (unsigned)std::max<int64_t>(1, std::min<int64_t>(2 * sms, (ls.P.n_items + per - 1) / per));
+  wgd::window_group_kernel<C><<<grid, wgd::kWinBlock, 0, st>>>(ls.P);
+  return true;
+}
+
+bool launch_window_static(const LaunchSpec& ls, int sms, cudaStream_t st) {
+  using namespace wgd;
+  if (ls.vec == 0) return false;  // unaligned columns or a selection
+  switch (ls.P.shape) {
+    case SHAPE_GROUPBY: return launch_window_t<ShapeGroupBy>(ls, sms, st);
+    case SHAPE_BATCH_I64: return launch_window_t<ShapeBatchI64>(ls, sms, st);
+    case SHAPE_BATCH_F64: return launch_window_t<ShapeBatchF64>(ls, sms, st);
+    case SHAPE_IPV4: return launch_window_t<ShapeIPv4>(ls, sms, st);
+    default: return false;
+  }
 }
 
 void launch_static_shape(const LaunchSpec& ls, cudaStream_t st) {

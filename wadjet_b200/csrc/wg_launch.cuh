@@ -24,6 +24,10 @@ struct LaunchSpec {
   wgd::TileCfg cfg{};
   int vec = 0;                // compiled shapes: rows per lane of the vector kernel (0 = one-row kernel)
   bool lc = false;            // no compiled shape, groups in shared memory: lowcard_kernel
+  bool win = false;           // groups of a key window in an HBM array (wg_window.cuh)
+  bool win_known = false;     // the window is [win_base, win_base + win_slots), else sampled
+  long long win_base = 0;
+  int64_t win_slots = 0;      // slots of the window's buffer
   bool stage = false;         // vector kernel with a shared table: the self-staged variant (1024 threads, 1 CTA/SM)
 };
 
@@ -109,5 +113,14 @@ void launch_static_shape(const LaunchSpec& ls, cudaStream_t st);
 int lowcard_threads(int ctas_per_sm);
 int lowcard_rows(int threads);
 void launch_lowcard(const LaunchSpec& ls, cudaStream_t st);
+
+// A key window's kernels (ls.win): the window and its empty slots, the rows of
+// a plan without a compiled shape, the groups into the table (wg_agg_lowcard.cu);
+// the rows of a compiled shape, false when the shape has no such kernel
+// (wg_agg_static.cu).
+void launch_window_begin(const LaunchSpec& ls, int sms, cudaStream_t st);
+void launch_window_rows(const LaunchSpec& ls, int sms, cudaStream_t st);
+void launch_window_fold(const LaunchSpec& ls, int sms, cudaStream_t st);
+bool launch_window_static(const LaunchSpec& ls, int sms, cudaStream_t st);
 
 }  // namespace wg

@@ -292,9 +292,15 @@ __device__ __forceinline__ void lc_value(const Plan& P, const LcRowSet& r, const
 
 // A key's slot in the CTA's key table, inserting it: [0, S) a regular key, S
 // the key equal to the empty pattern, S + 1 the NULL key; -1 when the table is
-// at its fill limit or the key outside a dense range.
-__device__ __forceinline__ int lc_slot(const Plan& P, unsigned long long* keys, unsigned long long k0,
+// at its fill limit or the key outside a dense range (or, with the groups in a
+// key window in HBM, outside the window or NULL).
+template <bool SH>
+__device__ __forceinline__ int lc_slot(const Plan& P, const KeyWindow& w, unsigned long long* keys, unsigned long long k0,
                                        unsigned long long k1, bool knull, int* s_groups, int s_limit) {
+  if (!SH) {
+    const unsigned long long d = k0 - (unsigned long long)w.base;
+    return !knull && d < w.n ? (int)d : -1;
+  }
   const int S = P.smem_slots, kw = P.L.key_words;
   if (kw == 0) return 0;
   if (knull) return S + 1;
@@ -361,8 +367,9 @@ static __device__ __noinline__ void lc_far_row(const Plan& P, int64_t row, int32
 
 // Group keys of the rows in `live` and their shared slots; returns the rows
 // that have one, `far` the rows that have none.
-__device__ __forceinline__ unsigned lc_keys(const Plan& P, const LcRowSet& r, const LcExprs& ev, unsigned live,
-                                            unsigned long long* keys, int (&slot)[kLcRows], unsigned& far, int* s_groups,
+template <bool SH>
+__device__ __forceinline__ unsigned lc_keys(const Plan& P, const KeyWindow& w, const LcRowSet& r, const LcExprs& ev,
+                                            unsigned live, unsigned long long* keys, int (&slot)[kLcRows], unsigned& far, int* s_groups,
                                             int s_limit) {
   const Layout& L = P.L;
   unsigned long long k0[kLcRows], k1[kLcRows];
@@ -396,21 +403,29 @@ __device__ __forceinline__ unsigned lc_keys(const Plan& P, const LcRowSet& r, co
   }
   far = 0;
   WG_LC_LIVE(u, live) {
-    slot[u] = lc_slot(P, keys, k0[u], k1[u], (knull >> u) & 1u, s_groups, s_limit);
+    slot[u] = lc_slot<SH>(P, w, keys, k0[u], k1[u], (knull >> u) & 1u, s_groups, s_limit);
     far |= slot[u] < 0 ? 1u << u : 0u;
   }
   return live & ~far;
 }
 
-// The updates of the rows in `live`, aggregate by aggregate (apply<NA, true>'s,
-// with 32-bit NULL counters); acc: the lane's copy of the accumulators.
+// The updates of the rows in `live`, aggregate by aggregate (apply<NA, SH>'s,
+// with 32-bit NULL counters in shared memory); acc: the lane's copy of the
+// accumulators (SH), or the window's slots past their key word.
+template <bool SH>
+__device__ __forceinline__ void lc_count(unsigned long long* p) {
+  if (SH) atomicAdd((unsigned*)p, 1u);
+  else atomicAdd(p, 1ULL);
+}
+
+template <bool SH>
 __device__ __forceinline__ void lc_update(const Plan& P, const LcRowSet& r, const LcExprs& ev, unsigned live,
                                           unsigned long long* acc, const int (&slot)[kLcRows]) {
   const Layout& L = P.L;
-  const int kw = L.key_words, aw = P.smem_sw;
+  const int kw = L.key_words, aw = SH ? P.smem_sw : L.slot_words;
   unsigned long long* t[kLcRows];  // the row's group, indexed like a slot (key words first)
-  WG_LC_EACH(u) t[u] = acc + slot[u] * aw - kw;
-  WG_LC_LIVE(u, live) atomicAdd((unsigned*)(t[u] + kw), 1u);
+  WG_LC_EACH(u) t[u] = acc + (int64_t)slot[u] * aw - kw;
+  WG_LC_LIVE(u, live) lc_count<SH>(t[u] + kw);
 #pragma unroll 1
   for (int a = 0; a < L.n_aggs; ++a) {
     const int kind = L.agg[a].kind, off = L.agg[a].off, noff = L.agg[a].null_off, vcol = L.agg[a].vcol;
@@ -418,12 +433,15 @@ __device__ __forceinline__ void lc_update(const Plan& P, const LcRowSet& r, cons
     LcVals v;
     lc_value(P, r, ev, vcol, live, v);
     if (noff >= 0) {
-      WG_LC_LIVE(u, live & v.null) atomicAdd((unsigned*)(t[u] + noff), 1u);
+      WG_LC_LIVE(u, live & v.null) lc_count<SH>(t[u] + noff);
     }
     const unsigned m = live & ~v.null;
     switch (kind) {
       case K_SUM_I64:
-        WG_LC_LIVE(u, m) smem_add_limbs((unsigned*)(t[u] + off), 2, v.lo[u], 0);
+        WG_LC_LIVE(u, m) {
+          if (SH) smem_add_limbs((unsigned*)(t[u] + off), 2, v.lo[u], 0);
+          else if (v.lo[u]) atomicAdd(t[u] + off, v.lo[u]);
+        }
         break;
       case K_SUM_F64: {
         const int cls = P.vcls[vcol];
@@ -435,7 +453,10 @@ __device__ __forceinline__ void lc_update(const Plan& P, const LcRowSet& r, cons
         break;
       }
       case K_SUM_DEC:
-        WG_LC_LIVE(u, m) smem_add_limbs((unsigned*)(t[u] + off), 4, v.lo[u], v.hi[u]);
+        WG_LC_LIVE(u, m) {
+          if (SH) smem_add_limbs((unsigned*)(t[u] + off), 4, v.lo[u], v.hi[u]);
+          else atomic_add128(t[u] + off, v.lo[u], v.hi[u]);
+        }
         break;
       case K_MIN_I64:
         WG_LC_LIVE(u, m) {
@@ -459,7 +480,15 @@ __device__ __forceinline__ void lc_update(const Plan& P, const LcRowSet& r, cons
           if (o > *(volatile unsigned long long*)(t[u] + off)) atomicMax(t[u] + off, o);
         }
         break;
-      default: break;  // COUNT; DECIMAL MIN / MAX do not take this kernel
+      case K_MIN_DEC: case K_MAX_DEC:  // 16-byte compare-and-swap: in HBM only
+        if (!SH) {
+          WG_LC_LIVE(u, m) {
+            if (kind == K_MIN_DEC) atomic_min128((U128*)(t[u] + off), v.lo[u], v.hi[u]);
+            else atomic_max128((U128*)(t[u] + off), v.lo[u], v.hi[u]);
+          }
+        }
+        break;
+      default: break;  // COUNT
     }
   }
 }
@@ -509,25 +538,36 @@ __device__ __forceinline__ void lc_flush(const Plan& P, const unsigned long long
   }
 }
 
-template <int NA>
+// SH: groups in the CTA's shared memory; otherwise in the launch's key window
+// (wg_window.cuh), nothing when it has none.
+template <int NA, bool SH>
 __global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_constant__ Plan P) {
   extern __shared__ __align__(16) unsigned long long sm[];
   __shared__ int s_groups;
   __shared__ unsigned long long s_init[WG_MAX_SLOT_WORDS];
+  KeyWindow win;
+  win.base = 0;
+  win.n = 0;
+  if (!SH) {
+    win = *P.win;
+    if (win.n == 0) return;
+  }
   const int S = P.smem_slots, kw = P.L.key_words, aw = P.smem_sw, R = P.smem_rep;
   const int key_words = P.gdense ? 0 : S * kw;
   unsigned long long* keys = sm;
   unsigned long long* acc = sm + key_words;
   const int s_limit = (S * 7) / 8;
-  if (threadIdx.x < (unsigned)P.L.slot_words) s_init[threadIdx.x] = P.L.init[threadIdx.x];
-  if (threadIdx.x == 0) s_groups = 0;
-  for (int i = threadIdx.x; i < key_words; i += blockDim.x) keys[i] = kw == 1 ? WG_EMPTY_KEY : ~0ULL;
-  __syncthreads();
-  fill_pattern(acc, (int64_t)R * (S + 2) * aw, aw, P.L.slot_words - kw, s_init + kw, threadIdx.x, blockDim.x);
-  __syncthreads();
+  if (SH) {
+    if (threadIdx.x < (unsigned)P.L.slot_words) s_init[threadIdx.x] = P.L.init[threadIdx.x];
+    if (threadIdx.x == 0) s_groups = 0;
+    for (int i = threadIdx.x; i < key_words; i += blockDim.x) keys[i] = kw == 1 ? WG_EMPTY_KEY : ~0ULL;
+    __syncthreads();
+    fill_pattern(acc, (int64_t)R * (S + 2) * aw, aw, P.L.slot_words - kw, s_init + kw, threadIdx.x, blockDim.x);
+    __syncthreads();
+  }
   Credit cr;
   const int lane = threadIdx.x & 31;
-  unsigned long long* mine = acc + (size_t)(lane & (R - 1)) * (S + 2) * aw;
+  unsigned long long* mine = SH ? acc + (size_t)(lane & (R - 1)) * (S + 2) * aw : P.wslots + kw;
   const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * (32 * kLcRows);
   const int jt = P.has_join ? (P.join.direct ? WG_JOIN_INNER : P.join.jtype) : WG_JOIN_INNER;
   for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * kLcRows); base < P.n_items;
@@ -568,8 +608,8 @@ __global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_con
       for (int e = 0; e < P.n_exprs; ++e) lc_eval(P, r, e, live, ev.v + e * kLcRows, ev.null[e]);
       int slot[kLcRows];
       unsigned far;
-      const unsigned have = lc_keys(P, r, ev, live, keys, slot, far, &s_groups, s_limit);
-      lc_update(P, r, ev, have, mine, slot);
+      const unsigned have = lc_keys<SH>(P, win, r, ev, live, keys, slot, far, &s_groups, s_limit);
+      lc_update<SH>(P, r, ev, have, mine, slot);
       if (far) {
         WG_LC_LIVE(u, far) lc_far_row(P, r.row(u), r.brow[u], &cr);
       }
@@ -581,8 +621,10 @@ __global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_con
       }
     }
   }
-  __syncthreads();
-  lc_flush<NA>(P, keys, acc, cr);
+  if (SH) {
+    __syncthreads();
+    lc_flush<NA>(P, keys, acc, cr);
+  }
   cr.release(P.T);
 }
 
