@@ -87,3 +87,46 @@ def test_lean_equals_the_hbm_table(ctx, monkeypatch, shape, values, keys, n):
         np.testing.assert_array_equal(np.isinf(g[0]), np.isinf(w[0]))
         fin = np.isfinite(w[0])
         assert (np.abs(g[0][fin] - w[0][fin]) <= 1e-10 * np.abs(w[0][fin])).all()
+
+
+@pytest.mark.parametrize("limit", [1024, 4096])
+def test_batched_lean_equals_the_hbm_table(ctx, limit):
+    """The same row loop for the work items of a batch: queries in shared tables of two CTAs per
+    SM or one, and queries in HBM beside them (a launch each), against a batch whose tables are
+    all in HBM. A result is read twice (the second without a run in between)."""
+    import torch
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(limit)
+    queries = []
+    for i, (keys, n, hint) in enumerate([("dense", 100_003, 4000), ("sparse", 40_001, 3000), ("outliers", 4097, 900),
+                                         ("empty", 129, 50), ("many", 150_001, 2000), ("sparse", 1, 16),
+                                         ("many", 70_000, 30_000), ("dense", 66_000, 4000)]):
+        val = _values("int", n, rng) if i % 2 == 0 else _values(["wide", "special", "float", "float"][i // 2], n, rng)
+        cols = [torch.from_numpy(x).cuda() for x in
+                (_keys(keys, n, rng).astype(np.int64), val, rng.integers(0, 10, n, dtype=np.int32))]
+        queries.append(dict(batch=wg.Batch([wg.Column(I64, cols[0]), wg.Column(I64 if i % 2 == 0 else F64, cols[1]),
+                                            wg.Column(I32, cols[2])]), group_by=[0], ndv_hint=hint,
+                            aggs=[wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1),
+                                  wg.AggColumn(wg.AGG_MIN, 1), wg.AggColumn(wg.AGG_MAX, 1)],
+                            filters=[(2, wg.OP_LT, 7)], keep=cols))
+    torch.cuda.synchronize()
+    out = []
+    for params in (wg.TuneParams(tile_rows=32768, smem_max_groups=limit), wg.TuneParams(smem_max_groups=-1)):
+        b = wg.BatchedQueries(ctx, queries, params)
+        for _ in range(2):  # the first run may re-run queries with more groups than their hint
+            counts = b.run()
+        res = [b.export(q, int(c)) for q, c in enumerate(counts)]
+        again = b.export(0, int(counts[0]))
+        np.testing.assert_array_equal(np.sort(again["keys"][0]), np.sort(res[0]["keys"][0]))
+        out.append(res)
+        b.close()
+    for i, (got, want) in enumerate(zip(*out)):
+        og, ow = canonical_order(got), canonical_order(want)
+        for f in ("keys", "count", "i64", "has"):
+            np.testing.assert_array_equal(got[f][:, og], want[f][:, ow])
+        g, w = got["f64"][:, og], want["f64"][:, ow]
+        np.testing.assert_array_equal(g[2:], w[2:])
+        np.testing.assert_array_equal(np.isnan(g[0]), np.isnan(w[0]))
+        np.testing.assert_array_equal(np.isinf(g[0]), np.isinf(w[0]))
+        fin = np.isfinite(w[0])
+        assert (np.abs(g[0][fin] - w[0][fin]) <= 1e-10 * np.abs(w[0][fin])).all()

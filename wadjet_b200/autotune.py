@@ -25,7 +25,7 @@ GRID = {
     "tile_rows": [8192, 32768, 131072],
     "block": [256, 512],
     "ctas_per_sm": [1, 2, 4],
-    "smem_max_groups": [-1, 1024, 8192],
+    "smem_max_groups": [-1, 1024, 4096],
     "max_load": [0.5],
 }
 
@@ -58,7 +58,7 @@ def sample_queries(ctx, nq: int, max_rows: int):
     return qs
 
 
-def time_params(ctx, qs, params, reps: int = 5) -> float:
+def time_params(ctx, qs, params, reps: int = 9) -> float:
     import torch
     import wadjet_b200 as wg
     b = wg.BatchedQueries(ctx, qs, params)

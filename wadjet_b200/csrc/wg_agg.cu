@@ -15,6 +15,7 @@
 #include "wg_internal.h"
 #include "wg_launch.cuh"
 #include "wg_hc.cuh"
+#include "wg_lean.cuh"
 
 #include <algorithm>
 #include <type_traits>
@@ -2407,7 +2408,7 @@ static wg_status spill_finish(wg_agg* a) {
 }
 
 // Compact the occupied slots once; the list drives export and emit.
-static wg_status agg_compact(wg_agg* a) {
+static wg_status launch_compact(wg_agg* a) {
   Ctx* ctx = a->ctx;
   const int64_t n = a->L.key_words == 0 ? 1 : (int64_t)a->cap + 2;
   WG_TRY(a->list.ensure(ctx, n * 8));
@@ -2417,8 +2418,13 @@ static wg_status agg_compact(wg_agg* a) {
                                                                   a->cnt.as<unsigned long long>());
   ctx->count_launch();
   WG_CUDA_TRY(cudaGetLastError());
+  return WG_OK;
+}
+
+static wg_status agg_compact(wg_agg* a) {
+  WG_TRY(launch_compact(a));
   int64_t c = 0;
-  WG_TRY(read_back_checked(ctx, a->cnt.as<int64_t>(), &c, 1));
+  WG_TRY(read_back_checked(a->ctx, a->cnt.as<int64_t>(), &c, 1));
   a->n_out = c;
   return WG_OK;
 }
@@ -3117,8 +3123,30 @@ __device__ __forceinline__ void batched_rows(const Plan& P, const Sh& sh, const 
   }
 }
 
+// A work item of a compiled shape with a shared table and vector-aligned
+// columns: the lean row loop (wg_lean.cuh), its sample taken per item. Each
+// form of an item is a call of its own: inlined together they spilled 764 bytes
+// at 64 registers, 100 apart. (64 queries of 16..4096 groups, 92.5M rows: 1.55 ms
+// with groups over 1024 in HBM, 0.83 now, all in shared memory; the columns take
+// 0.28 at the copy peak, and the last items of a launch leave SMs idle.)
+template <class C>
+__device__ __noinline__ void batched_lean(const Plan& P, const BatchItem& w, unsigned long long* sm, int* s_groups,
+                                             LeanSample* smp) {
+  constexpr bool kFixed = lean_float_sums<C>() > 0;  // the host sized the slots for it
+  Credit cr;
+  const int S = P.smem_slots;
+  smem_table_init(P, sm, S, s_groups);
+  lean_sample<C>(P, w.row0, w.row0 + w.rows, smp);
+  long long base = 0;
+  const bool dense = lean_run<C, kFixed>(P, w.row0, w.row0 + w.rows, threadIdx.x >> 5, blockDim.x >> 5, sm, S, *smp,
+                                         s_groups, &base, &cr);
+  __syncthreads();
+  smem_table_flush<C::n_aggs>(P, sm, S, cr, kFixed ? fixed_exponent_of(smp->exp) : 64, dense, base);
+  cr.release(P.T);
+}
+
 template <int NA, class Sh>
-__device__ __forceinline__ void batched_item(const Plan& P, const BatchItem& w, unsigned long long* sm,
+__device__ __noinline__ void batched_item(const Plan& P, const BatchItem& w, unsigned long long* sm,
                                              int* s_groups) {
   const Sh sh{P};
   Credit cr;  // reservations in this query's table, handed back before the next item
@@ -3136,13 +3164,14 @@ __device__ __forceinline__ void batched_item(const Plan& P, const BatchItem& w, 
 }
 
 // STATIC_ONLY: every query has a compiled shape, so the generic path (and its
-// registers) is left out and MB CTAs of 512 threads fit an SM.
+// registers) is left out. MB CTAs fill an SM's 1024 threads.
 template <int NA, bool STATIC_ONLY, int MB>
-__global__ void __launch_bounds__(512, MB) batched_kernel(const Plan* plans, const BatchItem* items, int64_t n_items,
+__global__ void __launch_bounds__(1024 / MB, MB) batched_kernel(const Plan* plans, const BatchItem* items, int64_t n_items,
                                                           unsigned long long* cursor) {
   extern __shared__ unsigned long long sm[];
   __shared__ int s_groups;
   __shared__ long long s_item;
+  __shared__ LeanSample s_smp;
   for (;;) {
     if (threadIdx.x == 0) s_item = (long long)atomicAdd(cursor, 1ULL);
     __syncthreads();
@@ -3150,9 +3179,14 @@ __global__ void __launch_bounds__(512, MB) batched_kernel(const Plan* plans, con
     if (it >= n_items) break;
     const BatchItem w = items[it];
     const Plan& P = plans[w.q];
+    const bool lean = P.vec_rows && P.smem_slots > 0;
     switch (P.shape) {
-      case SHAPE_BATCH_I64: batched_item<ShapeBatchI64::n_aggs, StatShape<ShapeBatchI64>>(P, w, sm, &s_groups); break;
-      case SHAPE_BATCH_F64: batched_item<ShapeBatchF64::n_aggs, StatShape<ShapeBatchF64>>(P, w, sm, &s_groups); break;
+      case SHAPE_BATCH_I64:
+        if (lean) { batched_lean<ShapeBatchI64>(P, w, sm, &s_groups, &s_smp); break; }
+        batched_item<ShapeBatchI64::n_aggs, StatShape<ShapeBatchI64>>(P, w, sm, &s_groups); break;
+      case SHAPE_BATCH_F64:
+        if (lean) { batched_lean<ShapeBatchF64>(P, w, sm, &s_groups, &s_smp); break; }
+        batched_item<ShapeBatchF64::n_aggs, StatShape<ShapeBatchF64>>(P, w, sm, &s_groups); break;
       default:
         if constexpr (!STATIC_ONLY) batched_item<NA, DynShape>(P, w, sm, &s_groups);
         break;
@@ -3180,8 +3214,21 @@ struct wg_batched {
   std::vector<ResetDesc> reset_h;
   wg::DevBuf plans, items, resets, cursor, counts;
   long long* counts_host = nullptr;
+  int launches = 0;
+  int64_t hbm_items = 0;     // the first items: queries without a shared table
+  bool counted = false;      // counts_host holds the last run's groups per query
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
+
+  // A table that takes more than half an SM's shared memory leaves room for one
+  // CTA: it then has twice the threads.
+  bool wide() const { return (int64_t)dyn_smem > (int64_t)ctx->max_smem_optin / 2 - 2048; }
+  int threads() const { return wide() ? 2 * tp.block : tp.block; }
+  using Kernel = void (*)(const wgd::Plan*, const BatchItem*, int64_t, unsigned long long*);
+  Kernel kernel(bool one_cta) const {
+    if (one_cta) return all_static ? batched_kernel<4, true, 1> : max_na <= 4 ? batched_kernel<4, false, 1> : batched_kernel<8, false, 1>;
+    return all_static ? batched_kernel<4, true, 2> : max_na <= 4 ? batched_kernel<4, false, 2> : batched_kernel<8, false, 2>;
+  }
 };
 
 namespace wg {
@@ -3214,28 +3261,42 @@ static wg_status batched_plan(wg_batched* b) {
     bool plain = a->L.key_words == 1;
     for (int i = 0; i < a->L.n_aggs; ++i)
       plain = plain && a->L.agg[i].null_off < 0 && a->L.agg[i].kind != wgd::K_MIN_DEC && a->L.agg[i].kind != wgd::K_MAX_DEC;
+    P.shape = pick_shape(P);
+    if (P.shape != wgd::SHAPE_BATCH_I64 && P.shape != wgd::SHAPE_BATCH_F64) P.shape = wgd::SHAPE_GENERIC;
+    // compiled shapes over 16-byte aligned columns take vector loads, and the lean
+    // row loop when the groups fit a shared table; the float shape's SUM then
+    // accumulates in two fixed-point words of the slot
+    {
+      bool vec = P.shape != wgd::SHAPE_GENERIC && !P.has_join && env_int("WG_BATCH_VEC", 1) != 0;
+      for (int j = 0; j < P.n_in; ++j) vec = vec && ((uintptr_t)P.in[j].data % 16 == 0);
+      P.vec_rows = vec ? 1 : 0;
+    }
+    int stride = a->L.slot_words;
+    if (P.vec_rows && P.shape == wgd::SHAPE_BATCH_I64) stride = wgd::lean_stride<wgd::ShapeBatchI64>(false);
+    if (P.vec_rows && P.shape == wgd::SHAPE_BATCH_F64) {
+      stride = wgd::lean_stride<wgd::ShapeBatchF64>(true);
+      P.smem_rep = -1;
+    }
+    P.smem_sw = stride;
     const int64_t smax = b->tp.smem_max_groups;
     int S = 0;
     if (plain && a->hint > 0 && a->hint <= smax) {
-      // at most the shared memory one CTA may take; a table that would then run
-      // more than 3/4 full stays in HBM
-      const int64_t fit = ((int64_t)ctx->max_smem_optin - 1024) / (a->L.slot_words * 8);
-      S = (int)std::min<int64_t>(fit, std::max<int64_t>(256, std::min<int64_t>(16384, a->hint * 2)));
-      if ((int64_t)S * 3 < a->hint * 4) S = 0;
-      max_smem_words = std::max<int64_t>(max_smem_words, (int64_t)S * a->L.slot_words);
+      // twice the groups while two CTAs share an SM, then up to the shared memory one
+      // CTA may take. The lean loop wants a slot per group (keys of a range need no
+      // more, and hashed ones without a slot go to the HBM table); the general loop's
+      // table stays in HBM when it would run more than 3/4 full.
+      const int64_t want = std::max<int64_t>(256, std::min<int64_t>(16384, a->hint * 2));
+      const int64_t half = ((int64_t)ctx->max_smem_optin / 2 - 2048) / (stride * 8);
+      const int64_t fit = ((int64_t)ctx->max_smem_optin - 1024) / (stride * 8);
+      S = (int)std::min<int64_t>(half, want);
+      if ((int64_t)S * 3 < a->hint * 4) S = (int)std::min<int64_t>(fit, want);
+      if (P.vec_rows ? S < a->hint : (int64_t)S * 3 < a->hint * 4) S = 0;
+      max_smem_words = std::max<int64_t>(max_smem_words, (int64_t)S * stride);
     }
     P.smem_slots = S;
     {
       const int mm = env_int("WG_MINMAX_TEST", -1);
       P.minmax_test = mm >= 0 ? (mm != 0) : (b->inputs[q].len >= 8 * std::max<int64_t>(a->hint, 1));
-    }
-    P.shape = pick_shape(P);
-    if (P.shape != wgd::SHAPE_BATCH_I64 && P.shape != wgd::SHAPE_BATCH_F64) P.shape = wgd::SHAPE_GENERIC;
-    // compiled shapes over 16-byte aligned columns take 2 rows per lane with vector loads
-    {
-      bool vec = P.shape != wgd::SHAPE_GENERIC && !P.has_join && env_int("WG_BATCH_VEC", 1) != 0;
-      for (int j = 0; j < P.n_in; ++j) vec = vec && ((uintptr_t)P.in[j].data % 16 == 0);
-      P.vec_rows = vec ? 1 : 0;
     }
     a->last_shape = P.shape;
     if (a->L.n_aggs > 4) b->max_na = 8;
@@ -3260,9 +3321,13 @@ static wg_status batched_plan(wg_batched* b) {
   for (int q = 0; q < n; ++q) order[q] = q;
   std::sort(order.begin(), order.end(), [&](int x, int y) { return b->inputs[x].len > b->inputs[y].len; });
   b->items_h.clear();
-  for (int q : order)
-    for (int64_t r0 = 0; r0 < b->inputs[q].len; r0 += b->tp.tile_rows)
-      b->items_h.push_back(BatchItem{q, (int32_t)std::min<int64_t>(b->tp.tile_rows, b->inputs[q].len - r0), r0});
+  for (int shared = 0; shared < 2; ++shared) {  // (the two launches of batched_enqueue)
+    for (int q : order)
+      if ((b->plans_h[q].smem_slots > 0) == (shared != 0))
+        for (int64_t r0 = 0; r0 < b->inputs[q].len; r0 += b->tp.tile_rows)
+          b->items_h.push_back(BatchItem{q, (int32_t)std::min<int64_t>(b->tp.tile_rows, b->inputs[q].len - r0), r0});
+    if (!shared) b->hbm_items = (int64_t)b->items_h.size();
+  }
   WG_TRY(b->items.ensure(ctx, (int64_t)(sizeof(BatchItem) * std::max<size_t>(1, b->items_h.size()))));
   if (!b->items_h.empty())
     WG_CUDA_TRY(cudaMemcpy(b->items.get(), b->items_h.data(), sizeof(BatchItem) * b->items_h.size(), cudaMemcpyHostToDevice));
@@ -3271,39 +3336,69 @@ static wg_status batched_plan(wg_batched* b) {
   return WG_OK;
 }
 
-static void batched_enqueue(wg_batched* b, cudaStream_t st) {
+// Queries without a shared table run in a launch of their own that leaves the
+// SMs' L1 whole: their probes and MIN/MAX tests hit it (16 queries of 1K-4K
+// groups: 770 us, and about 2 ms beside 113 KB tables in one launch). The other
+// queries' launch is a branch of the graph beside it and fills the SMs as its
+// CTAs leave.
+static wg_status batched_enqueue(wg_batched* b, cudaStream_t st, cudaStream_t st2, cudaEvent_t fork, cudaEvent_t join) {
   Ctx* ctx = b->ctx;
   const int n = (int)b->aggs.size();
   int64_t most = 1;
   for (const ResetDesc& r : b->reset_h) most = std::max(most, r.words);
   const dim3 rgrid((unsigned)n, (unsigned)std::min<int64_t>(64, (most + kResetWords - 1) / kResetWords));
   batched_reset_kernel<<<rgrid, kResetThreads, 0, st>>>(b->resets.as<ResetDesc>());
-  cudaMemsetAsync(b->cursor.get(), 0, 8, st);
+  WG_CUDA_TRY(cudaMemsetAsync(b->cursor.get(), 0, 16, st));
   const unsigned grid = (unsigned)(ctx->sm_count * std::max(1, b->tp.ctas_per_sm));
-  if (b->all_static) {
-    batched_kernel<4, true, 2><<<grid, b->tp.block, b->dyn_smem, st>>>(
-        b->plans.as<wgd::Plan>(), b->items.as<BatchItem>(), (int64_t)b->items_h.size(), b->cursor.as<unsigned long long>());
-  } else if (b->max_na <= 4) {
-    batched_kernel<4, false, 2><<<grid, b->tp.block, b->dyn_smem, st>>>(
-        b->plans.as<wgd::Plan>(), b->items.as<BatchItem>(), (int64_t)b->items_h.size(), b->cursor.as<unsigned long long>());
-  } else {
-    batched_kernel<8, false, 2><<<grid, b->tp.block, b->dyn_smem, st>>>(
-        b->plans.as<wgd::Plan>(), b->items.as<BatchItem>(), (int64_t)b->items_h.size(), b->cursor.as<unsigned long long>());
+  const wgd::Plan* plans = b->plans.as<wgd::Plan>();
+  const BatchItem* items = b->items.as<BatchItem>();
+  unsigned long long* cursor = b->cursor.as<unsigned long long>();
+  const int64_t shared_items = (int64_t)b->items_h.size() - b->hbm_items;
+  const bool both = b->hbm_items > 0 && shared_items > 0;
+  if (both) {
+    WG_CUDA_TRY(cudaEventRecord(fork, st));
+    WG_CUDA_TRY(cudaStreamWaitEvent(st2, fork, 0));
+  }
+  if (b->hbm_items > 0)
+    b->kernel(false)<<<grid, b->tp.block, 0, st>>>(plans, items, b->hbm_items, cursor);
+  if (shared_items > 0)
+    b->kernel(b->wide())<<<grid, b->threads(), b->dyn_smem, both ? st2 : st>>>(plans, items + b->hbm_items, shared_items,
+                                                                              cursor + 1);
+  WG_CUDA_TRY(cudaGetLastError());
+  if (both) {
+    WG_CUDA_TRY(cudaEventRecord(join, st2));
+    WG_CUDA_TRY(cudaStreamWaitEvent(st, join, 0));
   }
   batched_count_kernel<<<(n + 255) / 256, 256, 0, st>>>(b->resets.as<ResetDesc>(), n, b->counts.as<long long>());
-  cudaMemcpyAsync(b->counts_host, b->counts.get(), 8 * (size_t)n, cudaMemcpyDeviceToHost, st);
+  WG_CUDA_TRY(cudaMemcpyAsync(b->counts_host, b->counts.get(), 8 * (size_t)n, cudaMemcpyDeviceToHost, st));
+  b->launches = 2 + (b->hbm_items > 0) + (shared_items > 0);
+  return WG_OK;
 }
 
 static wg_status batched_capture(wg_batched* b) {
   Ctx* ctx = b->ctx;
   if (b->exec) { cudaGraphExecDestroy(b->exec); b->exec = nullptr; }
   if (b->graph) { cudaGraphDestroy(b->graph); b->graph = nullptr; }
-  WG_CUDA_TRY(cudaFuncSetAttribute(batched_kernel<4, true, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->dyn_smem));
-  WG_CUDA_TRY(cudaFuncSetAttribute(batched_kernel<4, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->dyn_smem));
-  WG_CUDA_TRY(cudaFuncSetAttribute(batched_kernel<8, false, 2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->dyn_smem));
-  WG_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
-  batched_enqueue(b, ctx->stream);
-  WG_CUDA_TRY(cudaStreamEndCapture(ctx->stream, &b->graph));
+  WG_CUDA_TRY(cudaFuncSetAttribute(b->kernel(b->wide()), cudaFuncAttributeMaxDynamicSharedMemorySize, (int)b->dyn_smem));
+  // the second branch's stream and events live for the capture only
+  cudaStream_t st2 = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  auto body = [&]() -> wg_status {
+    WG_CUDA_TRY(cudaStreamCreateWithFlags(&st2, cudaStreamNonBlocking));
+    WG_CUDA_TRY(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    WG_CUDA_TRY(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    WG_CUDA_TRY(cudaStreamBeginCapture(ctx->stream, cudaStreamCaptureModeThreadLocal));
+    const wg_status s = batched_enqueue(b, ctx->stream, st2, fork, join);
+    const cudaError_t e = cudaStreamEndCapture(ctx->stream, &b->graph);  // (also after an error, to leave the capture)
+    WG_TRY(s);
+    WG_CUDA_TRY(e);
+    return WG_OK;
+  };
+  const wg_status s = body();
+  if (st2) cudaStreamDestroy(st2);
+  if (fork) cudaEventDestroy(fork);
+  if (join) cudaEventDestroy(join);
+  WG_TRY(s);
   WG_CUDA_TRY(cudaGraphInstantiate(&b->exec, b->graph, 0));
   return WG_OK;
 }
@@ -3325,7 +3420,7 @@ wg_status wg_batched_create(wg_ctx* ctx, int32_t n, const wg_batched_query* qs, 
   if (tp.block <= 0) tp.block = 512;
   tp.block = std::max(64, std::min(512, tp.block & ~31));
   if (tp.ctas_per_sm <= 0) tp.ctas_per_sm = 2;
-  if (tp.smem_max_groups == 0) tp.smem_max_groups = 2048;  // negative: never use shared memory
+  if (tp.smem_max_groups == 0) tp.smem_max_groups = 4096;  // negative: never use shared memory
   if (tp.smem_max_groups < 0) tp.smem_max_groups = 0;
   if (tp.max_load <= 0.0 || tp.max_load > kMaxLoad) tp.max_load = 0.5;
   b->tp = tp;
@@ -3382,8 +3477,9 @@ wg_status wg_batched_run(wg_batched* b, int64_t* n_groups) {
   if (!b) return fail(WG_E_INVALID, "batched is NULL");
   Ctx* ctx = b->ctx;
   WG_TRY(ensure_device(ctx));
+  b->counted = false;
   WG_CUDA_TRY(cudaGraphLaunch(b->exec, ctx->stream));
-  ctx->count_launch(4);
+  ctx->count_launch(b->launches);
   WG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   WG_TRY(check_device_error(ctx));
   const int n = (int)b->aggs.size();
@@ -3409,6 +3505,7 @@ wg_status wg_batched_run(wg_batched* b, int64_t* n_groups) {
     WG_TRY(batched_plan(b));
     WG_TRY(batched_capture(b));
   }
+  b->counted = true;
   return WG_OK;
 }
 
@@ -3416,8 +3513,18 @@ wg_status wg_batched_export(wg_batched* b, int32_t q, const wg_group_export* out
   if (!b || q < 0 || q >= (int32_t)b->aggs.size()) return fail(WG_E_INVALID, "bad query index");
   wg_agg* a = b->aggs[q];
   a->finalized = false;
-  int64_t g = 0;
-  WG_TRY(wg_agg_finalize(a, &g));
+  if (a->resolved && b->counted && !a->hc && !a->spill) {
+    // the run counted the query's groups: the compaction and the export's
+    // kernels are queued together, one wait for both (64 queries: a wait, a
+    // copy and two pageable error words each less)
+    WG_TRY(ensure_device(b->ctx));
+    WG_TRY(launch_compact(a));
+    a->n_out = b->counts_host[q];
+  } else {
+    int64_t g = 0;
+    WG_TRY(wg_agg_finalize(a, &g));
+  }
+  a->finalized = true;
   wg_status s = wg_agg_export(a, out);
   a->finalized = false;
   return s;
