@@ -127,3 +127,46 @@ def test_known_range_of_a_join_payload(ctx, monkeypatch):
 
     _both(ctx, monkeypatch, ["sum_i", "count"], run)
     join.close()
+
+
+@pytest.mark.parametrize("left", [4 << 20, 96 << 10])
+def test_buffers_kept_for_speed_refuse_nothing(left):
+    """Under a budget the window and the result staging give way: another allocation gets the
+    window's memory, and a result that its two staging slots do not fit is read in smaller
+    chunks, exports and pages alike."""
+    import torch
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(left)
+    key = torch.from_numpy(rng.integers(0, 200_000, N)).cuda()
+    val = torch.from_numpy(rng.integers(-100, 100, N)).cuda()
+    cols = [wg.Column(I64, key), wg.Column(I64, val)]
+
+    def run(ctx):
+        a = wg.HashAggregate(ctx, [0], [wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1)],
+                             ndv_hint=200_000)
+        wg.run_pipeline(ctx, wg.Batch(cols), a, device=True)
+        a.finalize()
+        return a
+
+    def pages(a):
+        out = []
+        while (page := a.next(130_000)) is not None:
+            out.append([np.array(v) for v, _ in page])
+        return np.stack([np.concatenate(c) for c in zip(*out)])
+
+    with wg.Context(0) as ctx:
+        a = run(ctx)
+        want, want_pages = a.export(), pages(a)
+        a.close()
+    budget = 256 << 20
+    with wg.Context(0, hbm_budget=budget) as ctx:
+        a = run(ctx)
+        used = ctx.ledger()["used"]
+        ctx.reserve(budget - used + (8 << 20))  # more than is free: the window's memory is given up
+        ctx.reserve(budget - ctx.ledger()["used"] - left)
+        got, got_pages = a.export(), pages(a)
+        assert ctx.ledger()["peak"] <= budget
+        a.close()
+    assert_groups_equal(got, want, ["sum_i", "count"])
+    order = lambda p: p[:, np.argsort(p[0])]
+    np.testing.assert_array_equal(order(got_pages), order(want_pages))

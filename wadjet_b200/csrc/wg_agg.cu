@@ -554,13 +554,13 @@ struct wg_agg {
   std::vector<wg::DevBuf> sp_norm, sp_ok, sp_words, sp_okdev;
   // export staging (kept for the next export): every output field of a chunk
   // side by side on the device, read back in one copy through pinned memory
-  wg::DevBuf exp_dev;
+  wg::SpareBuf exp_dev;
   // the in-HBM key-hash reorder's copy of the input and its counters (kept for
   // the next query: allocating and freeing GBs per query costs milliseconds)
   std::vector<wg::DevBuf> part_bufs;
   wg::DevBuf part_counts, part_offs;
   // a key window (its bounds, then its slots from kWindowHeader bytes on), kept for the next launch
-  wg::DevBuf win_buf;
+  wg::SpareBuf win_buf;
   char* exp_host = nullptr;
   int64_t exp_host_bytes = 0;
   cudaEvent_t exp_ev[2] = {nullptr, nullptr};
@@ -906,7 +906,7 @@ static wg_status launch_pipeline(wg_agg* a, const LaunchSpec& ls, int64_t n_item
   P.shape = pick_shape(P);
   a->last_shape = P.shape;
   P.win = nullptr;
-  if (l2.win && n_items >= kWindowMinRows) {
+  if (l2.win && n_items >= kWindowMinRows && a->win_buf.get()) {
     // both the window kernel and the table kernel are queued; the sampled
     // window decides on the device which of them takes the rows
     P.win = a->win_buf.as<wgd::KeyWindow>();
@@ -2448,13 +2448,25 @@ static void fill_final_args(wg_agg* a, FinalArgs& A) {
 // second slot lets the next chunk's kernel and copy run meanwhile. The staging
 // stays with the aggregate (one column's result took two allocations, two
 // frees and two pageable copies before: ten of each for a five-column page).
-template <class Launch, class Take>
-static wg_status read_out(wg_agg* a, int64_t n, int64_t C, int64_t slot, Launch launch, Take take) {
+// layout(C) places a chunk's fields and gives the slot's bytes; where the
+// ledger has no room for the slots, one slot, then smaller chunks (of whole
+// validity words) are tried.
+template <class Layout, class Launch, class Take>
+static wg_status read_out(wg_agg* a, int64_t n, int64_t C, Layout layout, Launch launch, Take take) {
   Ctx* ctx = a->ctx;
-  const int64_t chunks = (n + C - 1) / C;
-  slot = (slot + 255) & ~int64_t(255);
-  const int64_t total = slot * std::min<int64_t>(chunks, 2);
-  WG_TRY(a->exp_dev.ensure(ctx, total));
+  int64_t chunks = (n + C - 1) / C, slot = (layout(C) + 255) & ~int64_t(255), slots = std::min<int64_t>(chunks, 2);
+  wg_status room = a->exp_dev.ensure(ctx, slot * slots);
+  while (room == WG_E_NOMEM && (slots > 1 || C > 64)) {
+    if (slots > 1) slots = 1;
+    else C = (C / 2 + 63) & ~int64_t(63);
+    chunks = (n + C - 1) / C;
+    slot = (layout(C) + 255) & ~int64_t(255);
+    room = a->exp_dev.ensure(ctx, slot * slots);
+    if (room == WG_OK) set_error("");
+  }
+  WG_TRY(room);
+  const int64_t total = slot * slots;
+  auto at = [&](int64_t k) { return slots > 1 ? (k & 1) * slot : 0; };
   if (a->exp_host_bytes < total + 256) {
     if (a->exp_host) cudaFreeHost(a->exp_host);
     a->exp_host = nullptr;
@@ -2470,11 +2482,11 @@ static wg_status read_out(wg_agg* a, int64_t n, int64_t C, int64_t slot, Launch 
   int32_t* err = (int32_t*)(a->exp_host + a->exp_host_bytes - 256);  // the device error word, with the last chunk
   auto enqueue = [&](int64_t k) -> wg_status {
     const int64_t c = std::min(C, n - k * C);
-    char* dev = a->exp_dev.as<char>() + (k & 1) * slot;
+    char* dev = a->exp_dev.as<char>() + at(k);
     const int64_t used = launch(k * C, c, dev);
     ctx->count_launch();
     WG_CUDA_TRY(cudaGetLastError());
-    WG_CUDA_TRY(cudaMemcpyAsync(a->exp_host + (k & 1) * slot, dev, (size_t)used, cudaMemcpyDeviceToHost, ctx->stream));
+    WG_CUDA_TRY(cudaMemcpyAsync(a->exp_host + at(k), dev, (size_t)used, cudaMemcpyDeviceToHost, ctx->stream));
     if (k == chunks - 1)
       WG_CUDA_TRY(cudaMemcpyAsync(err, ctx->dev_error, 4, cudaMemcpyDeviceToHost, ctx->stream));
     WG_CUDA_TRY(cudaEventRecord(a->exp_ev[k & 1], ctx->stream));
@@ -2482,10 +2494,11 @@ static wg_status read_out(wg_agg* a, int64_t n, int64_t C, int64_t slot, Launch 
   };
   wg_status st = enqueue(0);
   for (int64_t k = 0; k < chunks && st == WG_OK; ++k) {
-    if (k + 1 < chunks) st = enqueue(k + 1);
+    if (slots > 1 && k + 1 < chunks) st = enqueue(k + 1);
     const cudaError_t e = cudaEventSynchronize(a->exp_ev[k & 1]);
     if (e != cudaSuccess) return fail(WG_E_CUDA, std::string("result read-out: ") + cudaGetErrorString(e));
-    if (st == WG_OK) take(k * C, std::min(C, n - k * C), a->exp_host + (k & 1) * slot);
+    if (st == WG_OK) take(k * C, std::min(C, n - k * C), a->exp_host + at(k));
+    if (slots == 1 && st == WG_OK && k + 1 < chunks) st = enqueue(k + 1);
   }
   if (st != WG_OK) {
     cudaStreamSynchronize(ctx->stream);
@@ -2711,13 +2724,21 @@ wg_status wg_agg_export(wg_agg* a, const wg_group_export* o) {
   struct Field { void* dst; int blocks; int64_t es; int64_t off; };
   Field f[7] = {{o->keys, nk, 8, 0}, {o->key_valid, nk, 1, 0}, {o->count, na, 8, 0}, {o->i64, na, 8, 0},
                 {o->f64, na, 8, 0}, {o->dec, na, 16, 0}, {o->has, na, 1, 0}};
-  int64_t total = 0;
+  bool any = false;
   for (Field& x : f) {
-    if (!x.dst || x.blocks == 0) { x.dst = nullptr; continue; }
-    x.off = total;
-    total += (x.blocks * C * x.es + 255) & ~int64_t(255);
+    if (x.blocks == 0) x.dst = nullptr;
+    any = any || x.dst != nullptr;
   }
-  if (total == 0) return WG_OK;
+  if (!any) return WG_OK;
+  auto layout = [&](int64_t rows) {
+    int64_t total = 0;
+    for (Field& x : f) {
+      if (!x.dst) continue;
+      x.off = total;
+      total += (x.blocks * rows * x.es + 255) & ~int64_t(255);
+    }
+    return total;
+  };
   auto launch = [&](int64_t s0, int64_t c, char* dev) -> int64_t {
     A.keys = f[0].dst ? (int64_t*)(dev + f[0].off) : nullptr;
     A.key_valid = f[1].dst ? (uint8_t*)(dev + f[1].off) : nullptr;
@@ -2745,7 +2766,7 @@ wg_status wg_agg_export(wg_agg* a, const wg_group_export* o) {
         std::memcpy((char*)x.dst + (b * n + s0) * x.es, host + x.off + b * c * x.es, (size_t)(c * x.es));
     }
   };
-  return read_out(a, n, C, total, launch, take);
+  return read_out(a, n, C, layout, launch, take);
 }
 
 wg_status wg_agg_emit(wg_agg* a, int64_t start, int64_t max_rows, wg_column* out_cols, int64_t* n_out) {
@@ -2777,14 +2798,18 @@ wg_status wg_agg_emit(wg_agg* a, int64_t start, int64_t max_rows, wg_column* out
   const int64_t C = std::min<int64_t>(m, int64_t(1) << 16);
   const int ncol = nk + na;
   int64_t es[WG_MAX_KEYS + WG_MAX_AGGS], off[WG_MAX_KEYS + WG_MAX_AGGS], voff[WG_MAX_KEYS + WG_MAX_AGGS], total = 0;
-  for (int c = 0; c < ncol; ++c) {
-    es[c] = c < nk ? (class_of(a->key_types[c]) == WG_CLS_I32 ? 4 : 8) : 8;
-    off[c] = total;
-    total += (C * es[c] + 15) & ~int64_t(15);
-    voff[c] = total;
-    total += (C + 63) / 64 * 8;
-    total = (total + 15) & ~int64_t(15);
-  }
+  auto layout = [&](int64_t rows) {
+    total = 0;
+    for (int c = 0; c < ncol; ++c) {
+      es[c] = c < nk ? (class_of(a->key_types[c]) == WG_CLS_I32 ? 4 : 8) : 8;
+      off[c] = total;
+      total += (rows * es[c] + 15) & ~int64_t(15);
+      voff[c] = total;
+      total += (rows + 63) / 64 * 8;
+      total = (total + 15) & ~int64_t(15);
+    }
+    return total;
+  };
   if (ncol == 0) {
     *n_out = m;
     return check_device_error(ctx);
@@ -2813,7 +2838,7 @@ wg_status wg_agg_emit(wg_agg* a, int64_t start, int64_t max_rows, wg_column* out
       }
     }
   };
-  WG_TRY(read_out(a, m, C, total, launch, take));
+  WG_TRY(read_out(a, m, C, layout, launch, take));
   *n_out = m;
   return WG_OK;
 }

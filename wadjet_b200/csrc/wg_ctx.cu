@@ -1,5 +1,7 @@
 // wg_ctx.cu — context, HBM ledger, errors, host-batch staging.
 #include "wg_internal.h"
+
+#include <algorithm>
 #include "wg_device.cuh"
 
 #include <condition_variable>
@@ -191,6 +193,31 @@ bool drop_parked(Ctx* ctx) {
   return any;
 }
 
+bool drop_spares(Ctx* ctx) {
+  std::lock_guard<std::mutex> g(ctx->spare_mu);
+  bool any = false;
+  for (SpareBuf* b : ctx->spares) {
+    any = any || b->get() != nullptr;
+    b->reset();  // (cudaFree waits for queued work)
+  }
+  return any;
+}
+
+wg_status SpareBuf::ensure(Ctx* ctx, int64_t bytes) {
+  if (listed_ == nullptr) {
+    std::lock_guard<std::mutex> g(ctx->spare_mu);
+    ctx->spares.push_back(this);
+    listed_ = ctx;
+  }
+  return DevBuf::ensure(ctx, bytes);
+}
+
+SpareBuf::~SpareBuf() {
+  if (!listed_) return;
+  std::lock_guard<std::mutex> g(listed_->spare_mu);
+  listed_->spares.erase(std::find(listed_->spares.begin(), listed_->spares.end(), this));
+}
+
 thread_local std::string t_err;
 
 void set_error(const std::string& msg) { t_err = msg; }
@@ -210,15 +237,18 @@ wg_status DevBuf::alloc(Ctx* ctx, int64_t bytes) {
   reset();
   if (bytes <= 0) return WG_OK;
   int64_t rounded = (bytes + 255) & ~int64_t(255);
-  if (!ctx->ledger.reserve(rounded))
+  if (!ctx->ledger.reserve(rounded) && !(drop_spares(ctx) && ctx->ledger.reserve(rounded)))
     return fail(WG_E_NOMEM, "HBM ledger: memory budget exceeded (used=" + std::to_string(ctx->ledger.used()) +
                                 ", requested=" + std::to_string(rounded) +
                                 ", budget=" + std::to_string(ctx->ledger.budget()) + ")");
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, (size_t)rounded);
-  if (e == cudaErrorMemoryAllocation && drop_parked(ctx)) {
-    cudaGetLastError();
-    e = cudaMalloc(&p, (size_t)rounded);
+  if (e == cudaErrorMemoryAllocation) {
+    const bool parked = drop_parked(ctx);
+    if (drop_spares(ctx) || parked) {
+      cudaGetLastError();
+      e = cudaMalloc(&p, (size_t)rounded);
+    }
   }
   if (e != cudaSuccess) {
     ctx->ledger.release(rounded);
@@ -443,7 +473,7 @@ wg_status wg_ledger_stats(wg_ctx* c, int64_t* used, int64_t* peak, int64_t* budg
 
 wg_status wg_ledger_reserve(wg_ctx* c, int64_t bytes) {
   if (!c || bytes < 0) return fail(WG_E_INVALID, "bad ledger reservation");
-  if (!c->ledger.reserve(bytes)) return fail(WG_E_NOMEM, "HBM ledger: memory budget exceeded");
+  if (!c->ledger.reserve(bytes) && !(drop_spares(c) && c->ledger.reserve(bytes))) return fail(WG_E_NOMEM, "HBM ledger: memory budget exceeded");
   return WG_OK;
 }
 

@@ -107,6 +107,21 @@ class DevBuf {
   int64_t bytes_ = 0;
 };
 
+// A buffer kept between calls that its owner can do without (it checks get()
+// before each use): dropped when the ledger would refuse an allocation of its
+// context, so keeping it refuses nothing that ran without it.
+class SpareBuf : public DevBuf {
+ public:
+  SpareBuf() = default;
+  SpareBuf(const SpareBuf&) = delete;
+  SpareBuf& operator=(const SpareBuf&) = delete;
+  ~SpareBuf();
+  wg_status ensure(Ctx* ctx, int64_t bytes);
+
+ private:
+  Ctx* listed_ = nullptr;
+};
+
 // ---- context ---------------------------------------------------------------
 struct Ctx {
   int device = 0;
@@ -142,6 +157,8 @@ struct Ctx {
   };
   std::vector<Parked> parked;
   std::mutex park_mu;
+  std::vector<SpareBuf*> spares;  // of the context's objects
+  std::mutex spare_mu;
 
   explicit Ctx(int64_t budget, Ledger* parent = nullptr) : ledger(budget, parent) {}
   void count_launch(int n = 1) { launches.fetch_add(n); }
@@ -168,6 +185,7 @@ wg_status send_pieces(Ctx* ctx, const std::vector<HostPiece>& pieces, int64_t by
 wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out);
 void park_block(Ctx* ctx, DevBuf* b);
 bool drop_parked(Ctx* ctx);
+bool drop_spares(Ctx* ctx);  // whether any held memory
 
 wg_status ensure_device(Ctx* ctx);           // cudaSetDevice(ctx->device)
 wg_status read_back_i64(Ctx* ctx, const int64_t* dev, int64_t* out, int n);
