@@ -447,6 +447,7 @@ wg_status wg_ctx_destroy(wg_ctx* c) {
   }
   drop_parked(c);
   if (c->pinned) cudaFreeHost(c->pinned);
+  if (c->out_pinned) cudaFreeHost(c->out_pinned);
   if (c->host_scalar) cudaFreeHost(c->host_scalar);
   if (c->dev_scalar) cudaFree(c->dev_scalar);
   if (c->dev_error) cudaFree(c->dev_error);

@@ -150,6 +150,11 @@ struct Ctx {
   std::mutex stage_mu;
   DevBuf win[2];
   cudaEvent_t h2d_done[2] = {nullptr, nullptr};
+  // pinned staging of small results, made by the first one; an aggregate whose
+  // result is larger, or reads while another thread does, has its own
+  static constexpr int64_t kOutPinned = int64_t(1) << 20;
+  char* out_pinned = nullptr;
+  std::mutex out_mu;
   // device blocks kept for reuse (take_block / park_block)
   struct Parked {
     void* ptr;
