@@ -130,3 +130,68 @@ def test_batched_lean_equals_the_hbm_table(ctx, limit):
         np.testing.assert_array_equal(np.isinf(g[0]), np.isinf(w[0]))
         fin = np.isfinite(w[0])
         assert (np.abs(g[0][fin] - w[0][fin]) <= 1e-10 * np.abs(w[0][fin])).all()
+
+
+def _same_groups(got, want, floats):
+    """Groups equal to the HBM-table path's, by the bounds of the module's first lines."""
+    og, ow = canonical_order(got), canonical_order(want)
+    for f in ("keys", "count", "i64", "has"):
+        np.testing.assert_array_equal(got[f][:, og], want[f][:, ow])
+    g, w = got["f64"][:, og], want["f64"][:, ow]
+    np.testing.assert_array_equal(g[2:], w[2:])
+    if floats:
+        assert (np.abs(g[0] - w[0]) <= 1e-10 * np.abs(w[0])).all()
+
+
+def _ten_thousand(spread, n, rng):
+    return rng.integers(0, 10_000, n) * (1 if spread == "dense" else 0x1234567891)
+
+
+@pytest.mark.parametrize("hint", [16, 100])
+@pytest.mark.parametrize("keys", ["dense", "sparse"])
+@pytest.mark.parametrize("shape", ["groupby", "i64", "f64"])
+def test_hint_far_below_the_groups(ctx, monkeypatch, shape, keys, hint):
+    """A hint two orders below 10,000 groups: every CTA meets more keys than its table takes, so
+    the table reaches its limit and the probes of absent keys end there."""
+    import wadjet_b200 as wg
+    n = 400_003
+    rng = np.random.default_rng(hint)
+    cols = (_ten_thousand(keys, n, rng).astype(np.int64), _values("int" if shape == "i64" else "float", n, rng),
+            rng.integers(0, 10, n, dtype=np.int32))
+    monkeypatch.setenv("WG_AGG_SMEM", "1")
+    got = _run(ctx, wg, shape, cols, hint, n)
+    monkeypatch.setenv("WG_AGG_SMEM", "0")
+    _same_groups(got, _run(ctx, wg, shape, cols, hint, n), shape == "f64")
+
+
+@pytest.mark.parametrize("hint", [16, 100])
+@pytest.mark.parametrize("keys", ["dense", "sparse"])
+def test_batched_hint_far_below_the_groups(ctx, keys, hint):
+    """The same for work items, whose tables have 256 slots for such hints: first runs (the rows
+    of an item into its small table, then the query again alone) and the run after them."""
+    import torch
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(hint + 1)
+    queries = []
+    for i, n in enumerate([200_003, 90_001, 40_000]):
+        val = _values("int" if i % 2 == 0 else "float", n, rng)
+        cols = [torch.from_numpy(x).cuda() for x in
+                (_ten_thousand(keys, n, rng).astype(np.int64), val, rng.integers(0, 10, n, dtype=np.int32))]
+        queries.append(dict(batch=wg.Batch([wg.Column(I64, cols[0]), wg.Column(I64 if i % 2 == 0 else F64, cols[1]),
+                                            wg.Column(I32, cols[2])]), group_by=[0], ndv_hint=hint,
+                            aggs=[wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1),
+                                  wg.AggColumn(wg.AGG_MIN, 1), wg.AggColumn(wg.AGG_MAX, 1)],
+                            filters=[(2, wg.OP_LT, 7)], keep=cols))
+    torch.cuda.synchronize()
+    out = []
+    for params in (wg.TuneParams(tile_rows=32768), wg.TuneParams(smem_max_groups=-1)):
+        b = wg.BatchedQueries(ctx, queries, params)
+        res = []
+        for _ in range(2):
+            counts = b.run()
+            res.append([b.export(q, int(c)) for q, c in enumerate(counts)])
+        out.append(res)
+        b.close()
+    for got_run, want_run in zip(*out):
+        for i, (got, want) in enumerate(zip(got_run, want_run)):
+            _same_groups(got, want, i % 2 == 1)

@@ -43,6 +43,10 @@ constexpr int lean_stride(bool fixed) {
 }
 
 // Insert or find from slot h on: the slot's index, -1 when the table has no room for the key.
+// A thread reserves its place in *s_groups before it installs a key and gives it back when
+// another thread's key took the slot, so the table never holds more than s_limit < S keys: with
+// a check before and an add after, every thread between the two passes the limit, and a small
+// table (256 slots, 32 of them spare) fills.
 template <int SW>
 static __device__ __noinline__ int lean_insert(unsigned long long* sm, int S, unsigned long long k, uint32_t h, int* s_groups,
                                         int s_limit) {
@@ -53,11 +57,13 @@ static __device__ __noinline__ int lean_insert(unsigned long long* sm, int S, un
     if (cur == k) return (int)h;
     if (cur == WG_EMPTY_KEY) {
       if (*((volatile int*)s_groups) >= s_limit) return -1;
-      const unsigned long long old = atomicCAS(s, WG_EMPTY_KEY, k);
-      if (old == WG_EMPTY_KEY) {
-        atomicAdd(s_groups, 1);
-        return (int)h;
+      if (atomicAdd(s_groups, 1) >= s_limit) {
+        atomicSub(s_groups, 1);
+        return -1;
       }
+      const unsigned long long old = atomicCAS(s, WG_EMPTY_KEY, k);
+      if (old == WG_EMPTY_KEY) return (int)h;
+      atomicSub(s_groups, 1);
       if (old == k) return (int)h;
     }
     h = h + 1 == (uint32_t)S ? 0u : h + 1;
@@ -163,11 +169,13 @@ __device__ __forceinline__ void lean_rows(const Plan& P, int64_t begin, int64_t 
         int at = (int)h[u];
         if (!DENSE) {
           unsigned long long c = cur[u];
-          while (c != k && c != WG_EMPTY_KEY) {
+          while (c != k && c != WG_EMPTY_KEY) {  // at most once around the table
             at = at + 1 == S ? 0 : at + 1;
+            if (at == (int)h[u]) break;
             c = *((volatile unsigned long long*)(sm + at * SW));
           }
           if (c == WG_EMPTY_KEY) at = lean_insert<SW>(sm, S, k, (uint32_t)at, s_groups, s_limit);
+          else if (c != k) at = -1;
           if (at < 0) { far |= 1u << u; continue; }
         }
         Contrib<NA> c;
