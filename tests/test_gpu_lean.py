@@ -195,3 +195,78 @@ def test_batched_hint_far_below_the_groups(ctx, keys, hint):
     for got_run, want_run in zip(*out):
         for i, (got, want) in enumerate(zip(got_run, want_run)):
             _same_groups(got, want, i % 2 == 1)
+
+
+def _magnitudes(n, groups, rng):
+    """Keys and positive values, one power of two per group: 2^-1000, 2^-500, 1, 2^500 or 2^990."""
+    key = rng.integers(0, groups, n)
+    return key, np.ldexp(rng.random(n) + 0.5, np.array([-1000, -500, 0, 500, 990])[key % 5])
+
+
+def _sums_close(e, key, val, keep):
+    """Each group's SUM within the rounding of its rows' additions in any order."""
+    order = np.argsort(e["keys"][0])
+    want = np.zeros(key.max() + 1)
+    np.add.at(want, key[keep], val[keep])
+    np.testing.assert_array_equal(e["keys"][0][order], np.unique(key[keep]))
+    want = want[np.unique(key[keep])]
+    assert (np.abs(e["f64"][0][order] - want) <= 1e-10 * want).all()
+
+
+@pytest.mark.parametrize("groups", [7, 300])
+def test_groups_of_small_values_beside_huge_ones(ctx, monkeypatch, groups):
+    """Groups whose values underflow at the scale that another group's values set: they add in
+    binary64. Plain and batched; the scale may also come from a row that the filter drops."""
+    import torch
+    import wadjet_b200 as wg
+    monkeypatch.setenv("WG_AGG_SMEM", "1")
+    n = 50_003
+    rng = np.random.default_rng(groups)
+    key, val = _magnitudes(n, groups, rng)
+    filt = rng.integers(0, 10, n, dtype=np.int32)
+    filt[key % 5 == 4] = 9  # the huge values are dropped in the second query
+    for f in (np.zeros(n, np.int32), filt):
+        _sums_close(_run(ctx, wg, "f64", (key, val, f), 400, n), key, val, f < 7)
+    cols = [torch.from_numpy(x).cuda() for x in (key, val, filt)]
+    b = wg.BatchedQueries(ctx, [dict(batch=wg.Batch([wg.Column(I64, cols[0]), wg.Column(F64, cols[1]),
+                                                     wg.Column(I32, cols[2])]), group_by=[0], ndv_hint=400,
+                                     aggs=[wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1),
+                                           wg.AggColumn(wg.AGG_MIN, 1), wg.AggColumn(wg.AGG_MAX, 1)],
+                                     filters=[(2, wg.OP_LT, lim)]) for lim in (10, 7)])
+    counts = b.run()
+    for q, lim in enumerate((10, 7)):
+        _sums_close(b.export(q, int(counts[q])), key, val, filt < lim)
+    b.close()
+
+
+def test_star_join_small_products_beside_huge_ones(ctx):
+    """The same in the star join's SUM(price * (1 - disc)): products near 2^-152 in every group
+    but one, whose products near 2^1005 set the scale."""
+    import torch
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(6)
+    nd, n = 1 << 12, 40_003
+    grp = (np.arange(nd) % 50).astype(np.int32)
+    fk = rng.integers(0, nd, n).astype(np.int32)
+    huge = grp[fk] == 0
+    price = np.zeros(n, wg.DEC_DTYPE)  # units of 10^-30: 2^126 or 1
+    price["hi"], price["lo"] = np.where(huge, 1 << 62, 0), np.where(huge, 0, 1)
+    disc = np.where(huge, -(2.0 ** 979), 1.0 - 2.0 ** -53)
+    qty = np.full(n, 20, np.int32)
+    j = wg.HashJoin(ctx, 0, 0, payload=[1], build_row_hint=nd)
+    j.build([wg.Batch([wg.Column(I32, np.arange(nd, dtype=np.int32)), wg.Column(I32, grp)])])
+    g = wg.HashAggregate(ctx, [4], [wg.AggColumn(wg.AGG_SUM, 5), wg.AggColumn(wg.AGG_SUM, 2)], ndv_hint=50)
+    dev = [torch.from_numpy(x).cuda() for x in (fk, qty, price.view(np.int64).reshape(-1, 2), disc)]
+    batch = wg.Batch([wg.Column(I32, dev[0]), wg.Column(I32, dev[1]), wg.Column(17, dev[2], scale=30),
+                      wg.Column(F64, dev[3])])
+    wg.run_pipeline(ctx, batch, g, filters=[(1, wg.OP_GT, 10)], join=j, device=True,
+                    exprs=[wg.Expr(F64, [wg.Expr.col(2), wg.Expr.const_f(1.0), wg.Expr.col(3), "-", "*"])])
+    g.finalize()
+    assert g.kernel_shape == 1
+    e = g.export()
+    rows = np.bincount(grp[fk], minlength=50)
+    one = np.where(np.arange(50) == 0, float(1 << 126) / 1e30 * (1.0 + 2.0 ** 979), 1.0 / 1e30 * 2.0 ** -53)
+    want = (rows * one)[e["keys"][0]]
+    assert (np.abs(e["f64"][0] - want) <= 1e-10 * want).all()
+    g.close()
+    j.close()
