@@ -107,3 +107,60 @@ def test_joins(ctx, monkeypatch, jtype, key):
             return e
         _both(ctx, monkeypatch, run)
     join.close()
+
+
+@pytest.mark.parametrize("nulls", [False, True])
+@pytest.mark.parametrize("hint", [3700, 4000])
+def test_one_cta_table_then_an_outgrown_hint(ctx, monkeypatch, nulls, hint):
+    """Packed keys whose hint takes a whole SM's shared memory (5/8 to 3/4 of the slots), and
+    far more groups than the memory table was sized for: the overflow's replays."""
+    import wadjet_b200 as wg
+    n = 1_000_003
+    rng = np.random.default_rng(hint)
+    ok = rng.random(n) >= 0.1 if nulls else None
+    cols = [wg.Column(I32, rng.integers(0, 300, n, dtype=np.int32)), wg.Column(I32, rng.integers(0, 1000, n, dtype=np.int32)),
+            wg.Column(I64, rng.integers(-(1 << 40), 1 << 40, n), ok)]
+
+    def run():
+        a = wg.HashAggregate(ctx, [0, 1], [wg.AggColumn(wg.AGG_SUM, 2), wg.AggColumn(wg.AGG_COUNT, 2)], ndv_hint=hint)
+        wg.run_pipeline(ctx, wg.Batch(cols), a)
+        a.finalize()
+        e = a.export()
+        a.close()
+        return e
+
+    monkeypatch.setenv("WG_AGG_SMEM", "1")
+    got = run()
+    monkeypatch.setenv("WG_AGG_SMEM", "0")
+    assert_groups_equal(got, run(), ["sum_i", "count"])
+
+
+def test_row_counters_of_a_skewed_join_key(ctx, monkeypatch):
+    """One build key of 65,000 rows lets a CTA's share of the matches pass its 32-bit counters by
+    the worst case, so a plan whose table takes a whole SM's shared memory leaves it."""
+    import torch
+    import wadjet_b200 as wg
+    n, b, hot = 5_400_001, 4000, 65_000
+    rng = np.random.default_rng(4)
+    bkey = np.concatenate([np.arange(b), np.full(hot, b)]) * 977
+    join = wg.HashJoin(ctx, 0, 0, payload=[1], build_row_hint=b + hot)
+    join.build([wg.Batch([wg.Column(I64, bkey), wg.Column(I32, (np.arange(b + hot) % 7).astype(np.int32))])])
+    fkey = torch.from_numpy(rng.integers(0, b, n) * 977).cuda()
+    fkey[n // 2] = b * 977
+    keys = [torch.from_numpy(rng.integers(0, m, n, dtype=np.int32)).cuda() for m in (50, 70)]
+    val = torch.from_numpy(rng.integers(0, 1 << 40, n)).cuda()
+    batch = wg.Batch([wg.Column(I64, fkey), wg.Column(I32, keys[0]), wg.Column(I32, keys[1]), wg.Column(I64, val)])
+
+    def run():
+        a = wg.HashAggregate(ctx, [1, 2], [wg.AggColumn(wg.AGG_SUM, 3), wg.AggColumn(wg.AGG_COUNT, -1)], ndv_hint=3700)
+        wg.run_pipeline(ctx, batch, a, join=join, device=True)
+        a.finalize()
+        e = a.export()
+        a.close()
+        return e
+
+    monkeypatch.setenv("WG_AGG_SMEM", "1")
+    got = run()
+    monkeypatch.setenv("WG_AGG_SMEM", "0")
+    assert_groups_equal(got, run(), ["sum_i", "count"])
+    join.close()

@@ -1104,6 +1104,29 @@ static int64_t smem_rows_per_cta(int64_t n, int64_t groups) {
   return std::max<int64_t>(4096, (int64_t)(std::sqrt((double)n * (double)std::max<int64_t>(groups, 1)) / 4));
 }
 
+// The launch without a shared table, every field of it: the kernel's own
+// threads (a shared table that takes an SM has 1024, more than the generic
+// kernel is compiled for) and its grid. The tile kernel keeps its threads and grid.
+static void leave_shared(const Ctx* ctx, LaunchSpec& ls, bool stat, int blocks_per_sm) {
+  ls.smem = ls.lc = ls.stage = false;
+  ls.smem_bytes = 0;
+  ls.P.smem_slots = 0;
+  ls.P.gdense = 0;
+  if (ls.tile) return;
+  const int64_t n = ls.P.n_items;
+  if (!stat) {
+    ls.block = wgd::DynShape::kBlock;
+    ls.grid = (unsigned)std::min<int64_t>((int64_t)ctx->sm_count * 4, (n + 1023) / 1024 + 1);
+    return;
+  }
+  if (ls.vec && ls.block == 1024) ls.block = 768;
+  const int64_t rows = (int64_t)ls.block * (ls.vec ? ls.vec : 1);
+  ls.grid = (unsigned)std::min<int64_t>((int64_t)ctx->sm_count * blocks_per_sm, (n + rows - 1) / rows + 1);
+}
+
+// lowcard_kernel's key table takes this many groups: 3/4 of its slots.
+static bool lowcard_fits(int64_t groups, int64_t slots) { return groups * 4 <= slots * 3; }
+
 // Shared-memory launch of a plan without a compiled shape (lowcard_kernel), or
 // none (ls.smem false: the rows update the HBM table): the expected groups (or
 // the keys of a known range [glo, ghi]) must fit the key table at most 3/4
@@ -1114,10 +1137,7 @@ static int64_t smem_rows_per_cta(int64_t n, int64_t groups) {
 static void lowcard_setup(wg_agg* a, LaunchSpec& ls, int64_t expect, bool ranged, long long glo, long long ghi,
                           bool any_dec_minmax) {
   Ctx* ctx = a->ctx;
-  ls.smem = ls.lc = false;
-  ls.smem_bytes = 0;
-  ls.P.smem_slots = 0;
-  ls.P.gdense = 0;
+  leave_shared(ctx, ls, false, 0);
   const int kw = a->L.key_words;
   if (any_dec_minmax || (kw > 0 && expect <= 0) || env_int("WG_AGG_SMEM", 1) == 0) return;
   const int64_t aw = (a->L.slot_words - kw) | 1;  // an odd stride spreads the slots over the banks
@@ -1127,7 +1147,7 @@ static void lowcard_setup(wg_agg* a, LaunchSpec& ls, int64_t expect, bool ranged
     const int64_t key_bytes = kw == 0 || dense ? 0 : kw * 8;
     const int64_t fit = (budget - 2 * aw * 8) / (aw * 8 + key_bytes);  // slots beside one copy
     int64_t S = kw == 0 ? 1 : dense ? (int64_t)(ghi - glo + 1) : std::max<int64_t>(8, 2 * expect);
-    if (S > fit && !dense && kw > 0 && expect * 4 <= fit * 3) S = fit;
+    if (S > fit && !dense && kw > 0 && lowcard_fits(expect, fit)) S = fit;
     if (S > fit || S > 16384) continue;
     int R = 32;
     while (R > 1 && S * key_bytes + R * (S + 2) * aw * 8 > budget) R >>= 1;
@@ -1392,10 +1412,7 @@ static wg_status run_device(const PipelineRun& r) {
   // shared-table row counters are 32-bit: a CTA's share of the rows (of the
   // matches, in the kernel that walks chains) stays below 2^31
   if (ls.smem && n_items * (ls.lc ? fan : 1) / std::max<int64_t>(1, ls.grid) >= (int64_t(1) << 31)) {
-    ls.smem = false;
-    ls.lc = false;
-    ls.P.smem_slots = 0;
-    ls.smem_bytes = 0;
+    leave_shared(ctx, ls, stat, pref_bps);
   }
   // Groups beyond shared memory keyed by one integer: a key window, its range
   // known (an inner join's payload column, a dictionary's ids) or sampled
@@ -1417,7 +1434,6 @@ static wg_status run_device(const PipelineRun& r) {
       set_error("");  // no room for the window: the table as it is
     }
   }
-  const wgd::Plan base = ls.P;
   // the room the launch policy plans with: the table's limit less the
   // reservations threads may hold unused
   auto limit = [&]() { return (int64_t)((double)a->cap * kMaxLoad) - credit_slack(a); };
@@ -1510,24 +1526,14 @@ static wg_status run_device(const PipelineRun& r) {
       WG_TRY(rebuild_table(a, a->cap * 4, a->L));
       WG_TRY(refresh_groups(a));
       const int64_t expect2 = std::max<int64_t>(a->hint, a->known_groups);
-      if (ls.smem && !ls.P.gdense && !fits(expect2, ls.lc ? ls.P.smem_slots : S)) {
-        ls.smem = false;
-        ls.lc = false;
-        ls.P.smem_slots = 0;
-        ls.smem_bytes = 0;
-      }
+      if (ls.smem && !ls.P.gdense && !(ls.lc ? lowcard_fits(expect2, ls.P.smem_slots) : fits(expect2, S)))
+        leave_shared(ctx, ls, stat, pref_bps);
       if (table_words(a, a->cap) * 8 > kSnapshotMaxBytes) break;
     }
   }
   // 3) large table: chunks that each fit, growing between chunks
   WG_TRY(refresh_groups(a));
-  if (ls.smem) {
-    ls.smem = ls.lc = false;
-    ls.P.smem_slots = 0;
-    ls.smem_bytes = 0;
-    if (!ls.tile) ls.grid = (unsigned)(ctx->sm_count * 4);
-    if (!stat) ls.block = wgd::DynShape::kBlock;
-  }
+  if (ls.smem) leave_shared(ctx, ls, stat, pref_bps);
   int64_t done = 0;
   const int64_t min_chunk = 1 << 20;
   while (done < n_items) {
@@ -1541,8 +1547,7 @@ static wg_status run_device(const PipelineRun& r) {
     if (!ls.P.sel) m = std::max<int64_t>(64, m & ~int64_t(63));
     m = std::min<int64_t>(m, n_items - done);
     LaunchSpec lc = ls;
-    lc.P = base;
-    if (lc.P.sel) lc.P.sel = base.sel + done;
+    if (lc.P.sel) lc.P.sel = ls.P.sel + done;
     else rebase_cols(lc.P, done);
     WG_TRY(launch_pipeline(a, lc, m));
     WG_TRY(refresh_groups(a));
