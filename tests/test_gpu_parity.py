@@ -446,3 +446,32 @@ def test_shared_table_float_sums_across_the_fixed_point_range(ctx, n_keys):
     m.consume(ob.HostBatch([(I64, k, None, 0), (F64, np.abs(v), None, 0)]))
     assert_groups_equal(g.export(), o.export(), ["sum_f", "count"], magnitude=m.export())
     g.close()
+
+
+def test_a_refused_growth_leaves_the_aggregate_as_it_was():
+    """A batch whose groups need a larger table than the ledger has room for is refused; the
+    aggregate keeps the groups it had and takes the batch once there is room."""
+    import torch
+    import wadjet_b200 as wg
+    budget = 1 << 30
+    with wg.Context(0, hbm_budget=budget) as c:
+        small = torch.arange(1000, device="cuda")
+        large = torch.arange(600_000, device="cuda") * 7
+        aggs = [wg.AggColumn(wg.AGG_SUM, 0), wg.AggColumn(wg.AGG_COUNT, -1)]
+        g = wg.HashAggregate(c, [0], aggs, ndv_hint=16)
+        wg.run_pipeline(c, wg.Batch([wg.Column(I64, small)]), g, device=True)
+        held = budget - c.ledger()["used"] - (20 << 20)
+        c.reserve(held)
+        with pytest.raises(wg.MemoryExceeded):
+            wg.run_pipeline(c, wg.Batch([wg.Column(I64, large)]), g, device=True)
+        wg.run_pipeline(c, wg.Batch([wg.Column(I64, small)]), g, device=True)
+        c.release(held)
+        wg.run_pipeline(c, wg.Batch([wg.Column(I64, large)]), g, device=True)
+        g.finalize()
+        e = g.export()
+        order = np.argsort(e["keys"][0])
+        keys, rows = np.unique(np.concatenate([np.arange(1000)] * 2 + [np.arange(600_000) * 7]), return_counts=True)
+        np.testing.assert_array_equal(e["keys"][0][order], keys)
+        np.testing.assert_array_equal(e["count"][1][order], rows)
+        np.testing.assert_array_equal(e["i64"][0][order], keys * rows)
+        g.close()

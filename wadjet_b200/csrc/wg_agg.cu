@@ -695,18 +695,27 @@ static void run_fold(wg_agg* a, const wgd::Layout& Ls, const wgd::Table& Ts, con
 }
 
 // Re-create the table with capacity new_cap and/or a new layout, folding every
-// group across.
+// group across. Where memory is refused the aggregate keeps the table it has.
 static wg_status rebuild_table(wg_agg* a, uint64_t new_cap, const wgd::Layout& new_layout) {
   Ctx* ctx = a->ctx;
   const wgd::Layout old_L = a->L;
   const wgd::Table old_T = table_view(a);
-  DevBuf old_table = std::move(a->table);
-  DevBuf old_ctr = std::move(a->ctr);
+  const uint64_t old_cap = a->cap;
+  const int old_shift = a->shift;
   a->L = new_layout;
   a->cap = a->L.key_words == 0 ? 1 : new_cap;
   a->shift = 64 - log2u(a->cap);
-  WG_TRY(init_table(a, a->table, a->cap));
-  WG_TRY(a->ctr.alloc(ctx, 64));
+  DevBuf old_table, old_ctr;  // (the new ones until they are swapped in)
+  wg_status st = init_table(a, old_table, a->cap);
+  if (st == WG_OK) st = old_ctr.alloc(ctx, 64);
+  if (st != WG_OK) {
+    a->L = old_L;
+    a->cap = old_cap;
+    a->shift = old_shift;
+    return st;
+  }
+  std::swap(a->table, old_table);
+  std::swap(a->ctr, old_ctr);
   WG_CUDA_TRY(cudaMemsetAsync(a->ctr.get(), 0, 64, ctx->stream));
   wgd::Table old_view = old_T;
   old_view.slots = old_table.as<unsigned long long>();
@@ -853,8 +862,16 @@ static wg_status agg_check_nullable(wg_agg* a, const VSchema& vs) {
   build_layout(&tmp);
   for (int k = 0; k < WG_MAX_KEYS; ++k) tmp.L.key_vcol[k] = a->L.key_vcol[k];
   if (tmp.L.slot_words > WG_MAX_SLOT_WORDS) return fail(WG_E_UNSUPPORTED, "aggregate state too wide");
+  WG_TRY(rebuild_table(a, a->cap, tmp.L));
   a->nullable = nn;
-  return rebuild_table(a, a->cap, tmp.L);
+  return WG_OK;
+}
+
+// A reset that was refused its small table leaves none: the calls that would
+// read it fail until a reset gets one.
+static wg_status check_table(const wg_agg* a) {
+  if (a->table.get()) return WG_OK;
+  return fail(WG_E_NOMEM, "the aggregate's table was refused; reset it first");
 }
 
 static wg_status refresh_groups(wg_agg* a) {
@@ -1187,6 +1204,7 @@ static wg_status run_device(const PipelineRun& r) {
     a->hc = hc_eligible(r, ls.P);
     WG_TRY(agg_resolve(a, vs));
   } else {
+    WG_TRY(check_table(a));
     WG_TRY(agg_check_nullable(a, vs));
   }
   ls.P.err = ctx->dev_error;
@@ -2685,8 +2703,8 @@ wg_status wg_agg_merge(wg_agg* d, wg_agg* s) {
     tmp.key_cols = d->key_cols; tmp.specs = d->specs; tmp.kind = d->kind; tmp.nullable = nn; tmp.L = d->L;
     build_layout(&tmp);
     for (int k = 0; k < WG_MAX_KEYS; ++k) tmp.L.key_vcol[k] = d->L.key_vcol[k];
-    d->nullable = nn;
     WG_TRY(rebuild_table(d, d->cap, tmp.L));
+    d->nullable = nn;
   }
   WG_TRY(refresh_groups(d));
   int64_t s_groups = s->n_out;
@@ -2696,6 +2714,8 @@ wg_status wg_agg_merge(wg_agg* d, wg_agg* s) {
   }
   const int64_t need = d->known_groups + s_groups + credit_slack(d);
   if (d->L.key_words != 0 && need > (int64_t)((double)d->cap * kMaxLoad)) WG_TRY(rebuild_table(d, cap_for(need), d->L));
+  WG_TRY(check_table(d));
+  WG_TRY(check_table(s));
   run_fold(d, s->L, table_view(s), d->L, table_view(d), s->spilled ? s->n_out : -1,
            s->spilled ? s->list.as<int64_t>() : nullptr);
   WG_CUDA_TRY(cudaGetLastError());
@@ -2714,6 +2734,7 @@ wg_status wg_agg_finalize(wg_agg* a, int64_t* n_groups) {
     return WG_OK;
   }
   if (!a->finalized) {
+    WG_TRY(check_table(a));
     if (a->hc) WG_TRY(hc_finish(a));
     else if (a->spill) WG_TRY(spill_finish(a));
     else WG_TRY(agg_compact(a));  // its read-back checks the device error word
@@ -3022,6 +3043,7 @@ wg_status wg_agg_merge_state(wg_agg* a, const wg_state_layout* src, const void* 
     a->dom = 0;
     a->resolved = true;
   }
+  WG_TRY(check_table(a));
   if (a->L.key_words != src->key_words || a->kind != ref.kind)
     return fail(WG_E_INVALID, "aggregate input types differ");
   // the destination must carry every null counter the source has
@@ -3033,8 +3055,8 @@ wg_status wg_agg_merge_state(wg_agg* a, const wg_state_layout* src, const void* 
     tmp.key_cols = a->key_cols; tmp.specs = a->specs; tmp.kind = a->kind; tmp.nullable = nn; tmp.L = a->L;
     build_layout(&tmp);
     for (int k = 0; k < WG_MAX_KEYS; ++k) tmp.L.key_vcol[k] = a->L.key_vcol[k];
-    a->nullable = nn;
     WG_TRY(rebuild_table(a, a->cap, tmp.L));
+    a->nullable = nn;
   }
   if (n_rows == 0) return WG_OK;
   WG_TRY(refresh_groups(a));
