@@ -118,3 +118,42 @@ def test_batched_queries_with_joins_match_oracle(ctx):
         assert_groups_equal(bq.export(q, int(counts[q])), oracle_query(*h), kinds(h[3]))
     bq.close()
     join.close()
+
+
+def _by_key(e):
+    order = np.argsort(e["keys"][0])
+    return {f: e[f][:, order] for f in ("keys", "count", "i64", "has")}
+
+
+@pytest.mark.parametrize("jtype", ["inner", "semi"])
+def test_batched_outgrown_hint_keeps_its_join_and_projection(ctx, jtype):
+    """The run again of a query that outgrew its hint is the whole query: the join that drops
+    rows (and brings the key column, where it has a payload) and the projections."""
+    import torch
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(8)
+    n, nb = 200_003, 60_000
+    inner = jtype == "inner"
+    join = wg.HashJoin(ctx, 0, 0, payload=[1] if inner else [], build_row_hint=nb,
+                       join_type=wg.abi.JOIN_INNER if inner else wg.abi.JOIN_SEMI)
+    bkey = np.arange(nb) * 3
+    bgrp = (np.arange(nb) * 7).astype(np.int64)
+    join.build([wg.Batch([wg.Column(I64, bkey), wg.Column(I64, bgrp)])])
+    fk, val = rng.integers(0, 3 * nb, n), rng.integers(0, 1000, n)
+    cols = [torch.from_numpy(x).cuda() for x in (fk, val)]
+    q = dict(batch=wg.Batch([wg.Column(I64, cols[0]), wg.Column(I64, cols[1])]), group_by=[2 if inner else 0],
+             aggs=[wg.AggColumn(wg.AGG_SUM, 3 if inner else 2), wg.AggColumn(wg.AGG_COUNT, -1)], join=join,
+             exprs=[wg.Expr(I64, [wg.Expr.col(1), wg.Expr.const_i(5), "+"])], filters=[(1, wg.OP_LT, 900)], ndv_hint=16)
+    b = wg.BatchedQueries(ctx, [q])
+    keep = (val < 900) & (fk % 3 == 0)
+    key = bgrp[fk[keep] // 3] if inner else fk[keep]
+    uniq, at = np.unique(key, return_inverse=True)
+    for _ in range(2):  # the run that outgrows the table, and one on the grown table
+        counts = b.run()
+        assert counts[0] == len(uniq)
+        e = _by_key(b.export(0, int(counts[0])))
+        np.testing.assert_array_equal(e["keys"][0], uniq)
+        np.testing.assert_array_equal(e["i64"][0], np.bincount(at, val[keep] + 5).astype(np.int64))
+        np.testing.assert_array_equal(e["count"][1], np.bincount(at))
+    b.close()
+    join.close()

@@ -3556,7 +3556,8 @@ wg_status wg_batched_run(wg_batched* b, int64_t* n_groups) {
     // this query outgrew its hint: rerun it alone on a 4x table
     WG_TRY(rebuild_table(a, a->cap * 4, a->L));
     WG_TRY(wg_agg_reset(a));
-    PipelineRun r{a, &b->inputs[q], (int32_t)b->filters[q].size(), b->filters[q].data(), nullptr, 0, nullptr};
+    PipelineRun r{a, &b->inputs[q], (int32_t)b->filters[q].size(), b->filters[q].data(), b->joins[q],
+                  (int32_t)b->exprs[q].size(), b->exprs[q].data()};
     WG_TRY(run_device(r));
     int64_t g = 0;
     WG_TRY(wg_agg_finalize(a, &g));
