@@ -157,3 +157,35 @@ def test_batched_outgrown_hint_keeps_its_join_and_projection(ctx, jtype):
         np.testing.assert_array_equal(e["count"][1], np.bincount(at))
     b.close()
     join.close()
+
+
+def test_batched_run_after_a_refused_growth():
+    """Two queries outgrow their hints; the ledger has room for the first one's table and refuses
+    the second's. The next run, with room, runs on the tables there are."""
+    import torch
+    import wadjet_b200 as wg
+    rng = np.random.default_rng(2)
+    budget = 1 << 30
+    with wg.Context(0, hbm_budget=budget) as c:
+        qs, want = [], []
+        for n, distinct, hint in [(100_003, 20_000, 16), (900_001, 400_000, 100_000)]:
+            key, val = rng.integers(0, distinct, n) * 12345, rng.integers(0, 1000, n)
+            cols = [torch.from_numpy(x).cuda() for x in (key, val)]
+            qs.append(dict(batch=wg.Batch([wg.Column(I64, cols[0]), wg.Column(I64, cols[1])]), group_by=[0],
+                           aggs=[wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1)], ndv_hint=hint))
+            uniq, at = np.unique(key, return_inverse=True)
+            want.append((uniq, np.bincount(at, val).astype(np.int64), np.bincount(at)))
+        b = wg.BatchedQueries(c, qs, wg.TuneParams(max_load=0.5))
+        held = budget - c.ledger()["used"] - (25 << 20)  # the second table grown four times takes 25 MB beside the first
+        c.reserve(held)
+        with pytest.raises(wg.MemoryExceeded):
+            b.run()
+        c.release(held)
+        for _ in range(2):
+            counts = b.run()
+            for q, (keys, sums, rows) in enumerate(want):
+                e = _by_key(b.export(q, int(counts[q])))
+                np.testing.assert_array_equal(e["keys"][0], keys)
+                np.testing.assert_array_equal(e["i64"][0], sums)
+                np.testing.assert_array_equal(e["count"][1], rows)
+        b.close()

@@ -3282,6 +3282,7 @@ struct wg_batched {
   int launches = 0;
   int64_t hbm_items = 0;     // the first items: queries without a shared table
   bool counted = false;      // counts_host holds the last run's groups per query
+  bool moved = false;        // a table was replaced since the graph was captured
   cudaGraph_t graph = nullptr;
   cudaGraphExec_t exec = nullptr;
 
@@ -3543,17 +3544,26 @@ wg_status wg_batched_run(wg_batched* b, int64_t* n_groups) {
   Ctx* ctx = b->ctx;
   WG_TRY(ensure_device(ctx));
   b->counted = false;
+  // The graph names the tables' addresses: after a table was replaced it is captured
+  // again before it runs, also where an error ended the call that replaced it.
+  auto recapture = [&]() -> wg_status {
+    WG_TRY(batched_plan(b));
+    WG_TRY(batched_capture(b));
+    b->moved = false;
+    return WG_OK;
+  };
+  if (b->moved) WG_TRY(recapture());
   WG_CUDA_TRY(cudaGraphLaunch(b->exec, ctx->stream));
   ctx->count_launch(b->launches);
   WG_CUDA_TRY(cudaStreamSynchronize(ctx->stream));
   WG_TRY(check_device_error(ctx));
   const int n = (int)b->aggs.size();
-  bool replan = false;
   for (int q = 0; q < n; ++q) {
     wg_agg* a = b->aggs[q];
     a->finalized = false;
     if (b->counts_host[q] >= 0) continue;
     // this query outgrew its hint: rerun it alone on a 4x table
+    b->moved = true;
     WG_TRY(rebuild_table(a, a->cap * 4, a->L));
     WG_TRY(wg_agg_reset(a));
     PipelineRun r{a, &b->inputs[q], (int32_t)b->filters[q].size(), b->filters[q].data(), b->joins[q],
@@ -3563,14 +3573,10 @@ wg_status wg_batched_run(wg_batched* b, int64_t* n_groups) {
     WG_TRY(wg_agg_finalize(a, &g));
     a->finalized = false;
     b->counts_host[q] = g;
-    replan = true;
   }
   if (n_groups)
     for (int q = 0; q < n; ++q) n_groups[q] = b->counts_host[q];
-  if (replan) {  // tables moved: the graph must point at the new ones
-    WG_TRY(batched_plan(b));
-    WG_TRY(batched_capture(b));
-  }
+  if (b->moved) WG_TRY(recapture());
   b->counted = true;
   return WG_OK;
 }
