@@ -147,3 +147,31 @@ def test_fused_pipeline_with_bloom_matches_oracle(ctx, jt, monkeypatch):
     same groups as without it."""
     monkeypatch.setenv("WG_JOIN_BLOOM", "1")
     test_fused_pipeline_matches_oracle(ctx, jt, True, 0.05)
+
+
+@pytest.mark.parametrize("rows", [5000, 300_000])
+@pytest.mark.parametrize("smem", ["1", "0"])
+def test_group_by_a_payload_spread_over_all_64_bits(ctx, monkeypatch, smem, rows):
+    """Group keys that are an inner join's payload (hashes, say) whose smallest and largest value
+    lie further apart than a signed 64-bit difference holds: no dense table, window or bound
+    on the groups comes of such a range."""
+    import wadjet_b200 as wg
+    monkeypatch.setenv("WG_AGG_SMEM", smem)
+    rng = np.random.default_rng(rows)
+    pay = rng.integers(-(1 << 63), (1 << 63) - 1, rows)
+    pay[:2] = -(1 << 63) + 2, (1 << 63) - 1
+    join = wg.HashJoin(ctx, 0, 0, payload=[1], build_row_hint=rows)
+    join.build([wg.Batch([wg.Column(I64, np.arange(rows) * 11), wg.Column(I64, pay)])])
+    n = (1 << 20) + 5
+    at, val = rng.integers(0, rows, n), rng.integers(0, 1000, n)
+    a = wg.HashAggregate(ctx, [2], [wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1)], ndv_hint=3000)
+    wg.run_pipeline(ctx, wg.Batch([wg.Column(I64, at * 11), wg.Column(I64, val)]), a, join=join)
+    a.finalize()
+    e = a.export()
+    order = np.argsort(e["keys"][0])
+    uniq, back = np.unique(pay[at], return_inverse=True)
+    np.testing.assert_array_equal(e["keys"][0][order], uniq)
+    np.testing.assert_array_equal(e["i64"][0][order], np.bincount(back, val).astype(np.int64))
+    np.testing.assert_array_equal(e["count"][1][order], np.bincount(back))
+    a.close()
+    join.close()

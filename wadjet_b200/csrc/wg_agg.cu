@@ -1182,6 +1182,10 @@ static void lowcard_setup(wg_agg* a, LaunchSpec& ls, int64_t expect, bool ranged
   }
 }
 
+// Values of [lo, hi] less one, hi >= lo: a range of 64-bit values may span more
+// than a signed difference holds.
+static uint64_t span_of(long long lo, long long hi) { return (uint64_t)hi - (uint64_t)lo; }
+
 static wg_status run_device(const PipelineRun& r) {
   wg_agg* a = r.agg;
   Ctx* ctx = a->ctx;
@@ -1300,7 +1304,7 @@ static wg_status run_device(const PipelineRun& r) {
       ranged = true;
     }
     const bool cand = smem_ok && env_int("WG_GROUP_DENSE", 1) != 0 && a->L.n_keys == 1 && ranged && ghi >= glo &&
-                      ghi - glo < 16384;
+                      span_of(glo, ghi) < 16384;
     bool placed = false;
     for (int t = 0; t < 2 && cand && !placed; ++t) {
       if (t == 1 && (env_bps > 0 || pref_bps == 1)) break;
@@ -1425,7 +1429,7 @@ static wg_status run_device(const PipelineRun& r) {
     }
   }
 
-  if (!stat && !ls.tile) lowcard_setup(a, ls, expect, ranged && ghi - glo < 16384, glo, ghi, any_dec_minmax);
+  if (!stat && !ls.tile) lowcard_setup(a, ls, expect, ranged && ghi >= glo && span_of(glo, ghi) < 16384, glo, ghi, any_dec_minmax);
 
   // shared-table row counters are 32-bit: a CTA's share of the rows (of the
   // matches, in the kernel that walks chains) stays below 2^31
@@ -1439,7 +1443,7 @@ static wg_status run_device(const PipelineRun& r) {
   if (has_window && !ls.smem && !ls.tile && a->L.key_words == 1 && a->L.n_keys == 1 && !a->spill &&
       n_items >= kWindowMinRows && env_int("WG_KEY_WINDOW", 1) != 0) {
     const int64_t slot = (int64_t)a->L.slot_words * 8;
-    const bool known = ranged && ghi >= glo && (uint64_t)ghi - (uint64_t)glo < (uint64_t)(kWindowBytes / slot);
+    const bool known = ranged && ghi >= glo && span_of(glo, ghi) < (uint64_t)(kWindowBytes / slot);
     int64_t slots = 0;
     if (known) slots = ghi - glo + 1;
     else if (!r.join && expect > 0) slots = std::min<int64_t>(8 * std::max<int64_t>(expect, 1024), kWindowBytes / slot);
@@ -1468,7 +1472,7 @@ static wg_status run_device(const PipelineRun& r) {
     if (kv >= ls.P.n_in && kv < ls.P.n_in + npay && join_payload_range(r.join, kv - ls.P.n_in, &dlo, &dhi) &&
         dhi >= dlo) {
       if (a->dom == 1) { dlo = std::min(dlo, a->dom_lo); dhi = std::max(dhi, a->dom_hi); }
-      dom_ok = dhi - dlo < (int64_t(1) << 40);
+      dom_ok = span_of(dlo, dhi) < (uint64_t(1) << 40);
     }
   }
   if (r.str_ids && a->L.key_words == 1 && a->dom != 2) {
