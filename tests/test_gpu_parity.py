@@ -475,3 +475,19 @@ def test_a_refused_growth_leaves_the_aggregate_as_it_was():
         np.testing.assert_array_equal(e["count"][1][order], rows)
         np.testing.assert_array_equal(e["i64"][0][order], keys * rows)
         g.close()
+
+
+def test_emit_refuses_a_column_without_a_buffer(ctx):
+    """wg_agg_emit answers a NULL data pointer with an error, not with a write to it."""
+    import ctypes as C
+    import wadjet_b200 as wg
+    from wadjet_b200 import _abi as abi
+    a = wg.HashAggregate(ctx, [0], [wg.AggColumn(wg.AGG_COUNT, -1)], ndv_hint=16)
+    wg.run_pipeline(ctx, wg.Batch([wg.Column(I64, np.arange(10))]), a)
+    a.finalize()
+    key = np.zeros(10, np.int64)
+    cols = (abi.wg_column * 2)(abi.wg_column(I64, 0, key.ctypes.data, None, 10), abi.wg_column(I64, 0, None, None, 10))
+    n = C.c_int64(7)
+    assert wg.lib.wg_agg_emit(a.h, 0, 10, cols, C.byref(n)) != 0
+    assert n.value == 0
+    a.close()

@@ -2821,6 +2821,8 @@ wg_status wg_agg_emit(wg_agg* a, int64_t start, int64_t max_rows, wg_column* out
   *n_out = 0;
   if (start < 0 || start >= a->n_out || max_rows <= 0) return WG_OK;
   const int64_t m = std::min<int64_t>(max_rows, a->n_out - start);
+  for (int c = 0; c < nk + na; ++c)
+    if (!out_cols[c].data) return fail(WG_E_INVALID, "output column " + std::to_string(c) + " has no data buffer");
   if (!a->resolved) {  // scalar aggregate over no input: COUNT 0, everything else NULL
     for (int i = 0; i < na; ++i) {
       wg_column& c = out_cols[i];
