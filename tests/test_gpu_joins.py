@@ -175,3 +175,21 @@ def test_group_by_a_payload_spread_over_all_64_bits(ctx, monkeypatch, smem, rows
     np.testing.assert_array_equal(e["count"][1][order], np.bincount(back))
     a.close()
     join.close()
+
+
+def test_duplicate_keys_of_a_full_range_hold_no_payload_copy(ctx, monkeypatch):
+    """Build keys that fill a range but for a duplicate take the hash index, and hold no
+    more memory than where the payload copy of unique keys is never tried."""
+    import wadjet_b200 as wg
+    rows = 1 << 18
+    key = np.arange(rows, dtype=np.int32)
+    key[5] = 6
+    used = []
+    for full in ("0", "1"):
+        monkeypatch.setenv("WG_JOIN_FULL_DENSE", full)
+        before = ctx.ledger()["used"]
+        join = wg.HashJoin(ctx, 0, 0, payload=[1], build_row_hint=rows)
+        join.build([wg.Batch([wg.Column(I32, key), wg.Column(I32, key)])])
+        used.append(ctx.ledger()["used"] - before)
+        join.close()
+    assert used[0] == used[1]

@@ -994,7 +994,10 @@ static wg_status build_dense_unique(wg_join* j, bool* done) {
   WG_CUDA_TRY(cudaGetLastError());
   int64_t dup = 0;
   WG_TRY(read_back_checked(ctx, j->scratch.as<int64_t>() + kSwDup, &dup, 1));
-  if ((int32_t)dup != 0) return WG_OK;
+  if ((int32_t)dup != 0) {
+    j->dpay.reset();  // the hash index follows: its memory is not held against it
+    return WG_OK;
+  }
   j->pay_lo.assign(1, pay_int ? range_lo(back, 1) : 0);
   j->pay_hi.assign(1, pay_int ? range_hi(back, 1) : 0);
   j->pay_range.assign(1, pay_int);
