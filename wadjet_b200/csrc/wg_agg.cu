@@ -552,18 +552,12 @@ struct wg_agg {
   // packed words of a consume call; the flags' and words' staging at finalize
   std::vector<bool> sp_null;
   std::vector<wg::DevBuf> sp_norm, sp_ok, sp_words, sp_okdev;
-  // export staging (kept for the next export): every output field of a chunk
-  // side by side on the device, read back in one copy through pinned memory
-  wg::SpareBuf exp_dev;
   // the in-HBM key-hash reorder's copy of the input and its counters (kept for
   // the next query: allocating and freeing GBs per query costs milliseconds)
   std::vector<wg::DevBuf> part_bufs;
   wg::DevBuf part_counts, part_offs;
   // a key window (its bounds, then its slots from kWindowHeader bytes on), kept for the next launch
   wg::SpareBuf win_buf;
-  char* exp_host = nullptr;
-  int64_t exp_host_bytes = 0;
-  cudaEvent_t exp_ev[2] = {nullptr, nullptr};
   // Two-level partitioned mode (wg_hc.cuh), for tables far larger than L2:
   // each consume call writes its filtered rows, as the columns the aggregate
   // reads, to a first-level run in HBM; finalize re-partitions the runs into
@@ -587,9 +581,6 @@ struct wg_agg {
   wg::DevBuf hc_hll;                // distinct-key sketch of the rows consumed so far
   ~wg_agg() {
     for (auto& b : host_blocks) cudaFreeHost(b.first);
-    if (exp_host) cudaFreeHost(exp_host);
-    for (cudaEvent_t e : exp_ev)
-      if (e) cudaEventDestroy(e);
   }
 };
 
@@ -2469,76 +2460,52 @@ static void fill_final_args(wg_agg* a, FinalArgs& A) {
   }
 }
 
-// Rows [0, n) of the finalized groups to the host in chunks of C rows: launch
-// writes a chunk to `slot` bytes of device staging, which come back in one copy
-// into pinned staging, and take scatters them to the caller's arrays. A
-// second slot lets the next chunk's kernel and copy run meanwhile. The staging
-// stays with the aggregate (one column's result took two allocations, two
-// frees and two pageable copies before: ten of each for a five-column page).
-// layout(C) places a chunk's fields and gives the slot's bytes; where the
-// ledger has no room for the slots, one slot, then smaller chunks (of whole
-// validity words) are tried.
+// Rows [0, n) of the finalized groups to the host in chunks of at most C rows:
+// launch writes a chunk to the context's pinned block, and take scatters it to the
+// caller's arrays. Two halves of the block let the next chunk's kernel run
+// meanwhile. The kernels write to host memory themselves: no device staging,
+// nothing charged to the ledger, nothing that an aggregate pins for itself (a
+// new aggregate's first query used to pay for that).
+// layout(C) places a chunk's fields and gives their bytes.
 template <class Layout, class Launch, class Take>
 static wg_status read_out(wg_agg* a, int64_t n, int64_t C, Layout layout, Launch launch, Take take) {
   Ctx* ctx = a->ctx;
-  int64_t chunks = (n + C - 1) / C, slot = (layout(C) + 255) & ~int64_t(255), slots = std::min<int64_t>(chunks, 2);
-  wg_status room = a->exp_dev.ensure(ctx, slot * slots);
-  while (room == WG_E_NOMEM && (slots > 1 || C > 64)) {
-    if (slots > 1) slots = 1;
-    else C = (C / 2 + 63) & ~int64_t(63);
-    chunks = (n + C - 1) / C;
-    slot = (layout(C) + 255) & ~int64_t(255);
-    room = a->exp_dev.ensure(ctx, slot * slots);
-    if (room == WG_OK) set_error("");
+  std::lock_guard<std::mutex> reader(ctx->out_mu);  // (other readers' kernels run on the same stream)
+  if (!ctx->out_pinned && cudaMallocHost((void**)&ctx->out_pinned, Ctx::kOutPinned) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->out_pinned = nullptr;
+    return fail(WG_E_NOMEM, "pinned result staging allocation failed");
   }
-  WG_TRY(room);
-  const int64_t total = slot * slots;
-  auto at = [&](int64_t k) { return slots > 1 ? (k & 1) * slot : 0; };
-  char* host = nullptr;
-  std::unique_lock<std::mutex> shared(ctx->out_mu, std::defer_lock);
-  if (total + 256 <= Ctx::kOutPinned && shared.try_lock()) {
-    // (a new aggregate's first query of 2^20 rows, its result included: 4.3-4.6 ms with a block
-    // pinned for each aggregate, 1.5 with the context's)
-    if (!ctx->out_pinned && cudaMallocHost((void**)&ctx->out_pinned, Ctx::kOutPinned) != cudaSuccess) {
-      cudaGetLastError();
-      ctx->out_pinned = nullptr;
-      shared.unlock();
-    }
-    host = ctx->out_pinned;
-  }
-  if (!host && a->exp_host_bytes < total + 256) {
-    if (a->exp_host) cudaFreeHost(a->exp_host);
-    a->exp_host = nullptr;
-    a->exp_host_bytes = 0;
-    if (cudaMallocHost((void**)&a->exp_host, (size_t)total + 256) != cudaSuccess) {
-      cudaGetLastError();
-      return fail(WG_E_NOMEM, "pinned result staging allocation failed");
-    }
-    a->exp_host_bytes = total + 256;
-  }
-  if (!host) host = a->exp_host;
-  for (cudaEvent_t& e : a->exp_ev)
+  for (cudaEvent_t& e : ctx->out_ev)
     if (!e) WG_CUDA_TRY(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  int32_t* err = (int32_t*)(host + total);  // the device error word, with the last chunk
+  int32_t* err = (int32_t*)ctx->out_pinned;  // the device error word, with the last chunk
+  char* host = ctx->out_pinned + 256;
+  int64_t slot = Ctx::kOutPinned - 256;
+  C = std::min(C, n);
+  if (C < n || layout(C) > slot) {  // whole validity words per chunk
+    slot = (slot / 2) & ~int64_t(255);
+    C = std::max<int64_t>(64, (C + 63) & ~int64_t(63));
+    if (layout(C) > slot) C = std::max<int64_t>(64, (int64_t)((double)C * (double)slot / (double)layout(C)) & ~int64_t(63));
+    while (C > 64 && layout(C) > slot) C -= 64;
+  }
+  layout(C);
+  const int64_t chunks = (n + C - 1) / C;
+  auto at = [&](int64_t k) { return host + (k & 1) * (chunks > 1 ? slot : 0); };
   auto enqueue = [&](int64_t k) -> wg_status {
-    const int64_t c = std::min(C, n - k * C);
-    char* dev = a->exp_dev.as<char>() + at(k);
-    const int64_t used = launch(k * C, c, dev);
+    launch(k * C, std::min(C, n - k * C), at(k));
     ctx->count_launch();
     WG_CUDA_TRY(cudaGetLastError());
-    WG_CUDA_TRY(cudaMemcpyAsync(host + at(k), dev, (size_t)used, cudaMemcpyDeviceToHost, ctx->stream));
     if (k == chunks - 1)
       WG_CUDA_TRY(cudaMemcpyAsync(err, ctx->dev_error, 4, cudaMemcpyDeviceToHost, ctx->stream));
-    WG_CUDA_TRY(cudaEventRecord(a->exp_ev[k & 1], ctx->stream));
+    WG_CUDA_TRY(cudaEventRecord(ctx->out_ev[k & 1], ctx->stream));
     return WG_OK;
   };
   wg_status st = enqueue(0);
   for (int64_t k = 0; k < chunks && st == WG_OK; ++k) {
-    if (slots > 1 && k + 1 < chunks) st = enqueue(k + 1);
-    const cudaError_t e = cudaEventSynchronize(a->exp_ev[k & 1]);
+    if (k + 1 < chunks) st = enqueue(k + 1);
+    const cudaError_t e = cudaEventSynchronize(ctx->out_ev[k & 1]);
     if (e != cudaSuccess) return fail(WG_E_CUDA, std::string("result read-out: ") + cudaGetErrorString(e));
-    if (st == WG_OK) take(k * C, std::min(C, n - k * C), host + at(k));
-    if (slots == 1 && st == WG_OK && k + 1 < chunks) st = enqueue(k + 1);
+    if (st == WG_OK) take(k * C, std::min(C, n - k * C), at(k));
   }
   if (st != WG_OK) {
     cudaStreamSynchronize(ctx->stream);
@@ -2782,7 +2749,7 @@ wg_status wg_agg_export(wg_agg* a, const wg_group_export* o) {
     }
     return total;
   };
-  auto launch = [&](int64_t s0, int64_t c, char* dev) -> int64_t {
+  auto launch = [&](int64_t s0, int64_t c, char* dev) {
     A.keys = f[0].dst ? (int64_t*)(dev + f[0].off) : nullptr;
     A.key_valid = f[1].dst ? (uint8_t*)(dev + f[1].off) : nullptr;
     A.count = f[2].dst ? (int64_t*)(dev + f[2].off) : nullptr;
@@ -2794,12 +2761,6 @@ wg_status wg_agg_export(wg_agg* a, const wg_group_export* o) {
     A.n = c;
     A.stride = c;
     export_kernel<<<grid_cap(ctx, c, 256), 256, 0, ctx->stream>>>(A);
-    // the chunk's fields sit at their offsets with block stride c: up to the
-    // end of the last field in use
-    int64_t used = 0;
-    for (const Field& x : f)
-      if (x.dst) used = x.off + x.blocks * c * x.es;
-    return used;
   };
   auto take = [&](int64_t s0, int64_t c, const char* host) {
     // block b of the chunk (c rows at stride c) to rows [s0, s0 + c) of block b on the host (stride n)
@@ -2859,7 +2820,7 @@ wg_status wg_agg_emit(wg_agg* a, int64_t start, int64_t max_rows, wg_column* out
     *n_out = m;
     return check_device_error(ctx);
   }
-  auto launch = [&](int64_t s0, int64_t c, char* dev) -> int64_t {
+  auto launch = [&](int64_t s0, int64_t c, char* dev) {
     for (int k = 0; k < ncol; ++k) {
       A.out[k] = dev + off[k];
       A.out_valid[k] = (uint32_t*)(dev + voff[k]);
@@ -2867,7 +2828,6 @@ wg_status wg_agg_emit(wg_agg* a, int64_t start, int64_t max_rows, wg_column* out
     A.start = start + s0;
     A.n = c;
     emit_kernel<<<grid_cap(ctx, c, 256), 256, 0, ctx->stream>>>(A);
-    return total;
   };
   auto take = [&](int64_t s0, int64_t c, const char* host) {
     for (int k = 0; k < ncol; ++k) {

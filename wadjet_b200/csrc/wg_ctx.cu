@@ -448,6 +448,8 @@ wg_status wg_ctx_destroy(wg_ctx* c) {
   drop_parked(c);
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->out_pinned) cudaFreeHost(c->out_pinned);
+  for (cudaEvent_t e : c->out_ev)
+    if (e) cudaEventDestroy(e);
   if (c->host_scalar) cudaFreeHost(c->host_scalar);
   if (c->dev_scalar) cudaFree(c->dev_scalar);
   if (c->dev_error) cudaFree(c->dev_error);

@@ -150,10 +150,10 @@ struct Ctx {
   std::mutex stage_mu;
   DevBuf win[2];
   cudaEvent_t h2d_done[2] = {nullptr, nullptr};
-  // pinned staging of small results, made by the first one; an aggregate whose
-  // result is larger, or reads while another thread does, has its own
+  // pinned staging of results, made by the first one; the reader holds out_mu
   static constexpr int64_t kOutPinned = int64_t(1) << 20;
   char* out_pinned = nullptr;
+  cudaEvent_t out_ev[2] = {nullptr, nullptr};
   std::mutex out_mu;
   // device blocks kept for reuse (take_block / park_block)
   struct Parked {
