@@ -170,3 +170,93 @@ def test_buffers_kept_for_speed_refuse_nothing(left):
     assert_groups_equal(got, want, ["sum_i", "count"])
     order = lambda p: p[:, np.argsort(p[0])]
     np.testing.assert_array_equal(order(got_pages), order(want_pages))
+
+
+def _wide_query(wg, rng):
+    """Rows whose 200,000 groups take a key window, and the groups they give."""
+    import torch
+    key, val = rng.integers(0, 200_000, N), rng.integers(-100, 100, N)
+    keep = [torch.from_numpy(key).cuda(), torch.from_numpy(val).cuda()]
+    uniq, at = np.unique(key, return_inverse=True)
+    want = dict(keys=uniq, i64=np.bincount(at, val).astype(np.int64), count=np.bincount(at))
+    return wg.Batch([wg.Column(I64, keep[0]), wg.Column(I64, keep[1])]), keep, want
+
+
+def _equal(e, want):
+    order = np.argsort(e["keys"][0])
+    np.testing.assert_array_equal(e["keys"][0][order], want["keys"])
+    np.testing.assert_array_equal(e["i64"][0][order], want["i64"])
+    np.testing.assert_array_equal(e["count"][1][order], want["count"])
+
+
+def test_kept_buffers_of_two_threads():
+    """One context, two threads with an aggregate each, and a third whose reservations make the
+    context give its kept buffers back: a buffer in use stays its user's. A query that another
+    thread's reservation leaves no room says so; every other result is exact."""
+    import threading
+    import wadjet_b200 as wg
+    budget = 512 << 20
+    with wg.Context(0, hbm_budget=budget) as ctx:
+        batch, keep, want = _wide_query(wg, np.random.default_rng(5))
+        stop, errors, good = threading.Event(), [], [0, 0]
+
+        def query(i):
+            try:
+                for _ in range(25):
+                    a = wg.HashAggregate(ctx, [0], [wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1)],
+                                         ndv_hint=200_000)
+                    try:
+                        wg.run_pipeline(ctx, batch, a, device=True)
+                        a.finalize()
+                        e = a.export()
+                    except wg.MemoryExceeded:
+                        continue
+                    finally:
+                        a.close()
+                    _equal(e, want)
+                    good[i] += 1
+            except BaseException as x:  # noqa: BLE001
+                errors.append(x)
+
+        def squeeze():
+            while not stop.is_set():
+                n = budget - ctx.ledger()["used"] + (1 << 20)
+                try:
+                    ctx.reserve(n)
+                    ctx.release(n)
+                except wg.MemoryExceeded:
+                    pass
+                stop.wait(0.002)
+
+        threads = [threading.Thread(target=query, args=(i,)) for i in range(2)]
+        third = threading.Thread(target=squeeze)
+        for t in threads + [third]:
+            t.start()
+        for t in threads:
+            t.join()
+        stop.set()
+        third.join()
+        assert not errors, errors[0]
+        assert sum(good) >= 10
+        ctx.synchronize()
+        assert ctx.ledger()["peak"] <= budget
+
+
+def test_a_server_gives_its_slots_buffers_back():
+    """What a server's slots keep is charged to the budget they share, and gives way to a
+    reservation of the server's context."""
+    import wadjet_b200 as wg
+    budget = 1 << 30
+    with wg.Context(0, hbm_budget=budget) as ctx:
+        batch, keep, want = _wide_query(wg, np.random.default_rng(6))
+        s = wg.Server(ctx, 2)
+        tickets = [s.submit(batch=batch, group_by=[0], aggs=[wg.AggColumn(wg.AGG_SUM, 1), wg.AggColumn(wg.AGG_COUNT, -1)],
+                            ndv_hint=200_000) for _ in range(4)]
+        for t in tickets:
+            n, _ = s.wait(t, timeout=60.0)
+            _equal(s.export(t, n), want)
+            s.release(t)
+        free = budget - ctx.ledger()["used"]
+        ctx.reserve(free + (16 << 20))
+        ctx.release(free + (16 << 20))
+        s.close()

@@ -556,8 +556,6 @@ struct wg_agg {
   // the next query: allocating and freeing GBs per query costs milliseconds)
   std::vector<wg::DevBuf> part_bufs;
   wg::DevBuf part_counts, part_offs;
-  // a key window (its bounds, then its slots from kWindowHeader bytes on), kept for the next launch
-  wg::SpareBuf win_buf;
   // Two-level partitioned mode (wg_hc.cuh), for tables far larger than L2:
   // each consume call writes its filtered rows, as the columns the aggregate
   // reads, to a first-level run in HBM; finalize re-partitions the runs into
@@ -816,7 +814,7 @@ static wg_status agg_resolve(wg_agg* a, const VSchema& vs) {
   if (st == WG_E_NOMEM && a->L.key_words >= 1 && a->ctx->pinned_spill_bytes > 0 && env_int("WG_AGG_SPILL", 1) != 0) {
     // spill: one small table per hash partition, each holding about 1/16 of
     // what the ledger has left
-    const int64_t left = a->ctx->ledger.budget() > 0 ? a->ctx->ledger.budget() - a->ctx->ledger.used() : (int64_t(1) << 40);
+    const int64_t left = hbm_room(a->ctx);
     const int64_t full = (int64_t)a->cap * a->L.slot_words * 8;
     int pbits = 1;
     while (pbits < 10 && (full >> pbits) > left / 16) ++pbits;
@@ -914,16 +912,23 @@ static wg_status launch_pipeline(wg_agg* a, const LaunchSpec& ls, int64_t n_item
   P.shape = pick_shape(P);
   a->last_shape = P.shape;
   P.win = nullptr;
-  if (l2.win && n_items >= kWindowMinRows && a->win_buf.get()) {
+  // a key window: its bounds, then its slots from kWindowHeader bytes on; where
+  // memory has no room for it, the table as it is
+  DevBuf win;
+  if (l2.win && n_items >= kWindowMinRows) {
+    if (take_block(ctx, kWindowHeader + l2.win_slots * l2.P.L.slot_words * 8, &win) != WG_OK) set_error("");
+  }
+  if (win.get()) {
     // both the window kernel and the table kernel are queued; the sampled
     // window decides on the device which of them takes the rows
-    P.win = a->win_buf.as<wgd::KeyWindow>();
-    P.wslots = a->win_buf.as<unsigned long long>() + kWindowHeader / 8;
+    P.win = win.as<wgd::KeyWindow>();
+    P.wslots = win.as<unsigned long long>() + kWindowHeader / 8;
     launch_window_begin(l2, ctx->sm_count, ctx->stream);
     if (!launch_window_static(l2, ctx->sm_count, ctx->stream)) launch_window_rows(l2, ctx->sm_count, ctx->stream);
     if (!l2.win_known) launch_pipeline_shape(l2, ctx->stream);
     launch_window_fold(l2, ctx->sm_count, ctx->stream);
     ctx->count_launch(l2.win_known ? 4 : 5);
+    park_block(ctx, &win);  // its uses are queued on the context's stream
     WG_CUDA_TRY(cudaGetLastError());
     return WG_OK;
   }
@@ -1438,14 +1443,10 @@ static wg_status run_device(const PipelineRun& r) {
     int64_t slots = 0;
     if (known) slots = ghi - glo + 1;
     else if (!r.join && expect > 0) slots = std::min<int64_t>(8 * std::max<int64_t>(expect, 1024), kWindowBytes / slot);
-    if (slots > 0 && a->win_buf.ensure(ctx, kWindowHeader + slots * slot) == WG_OK) {
-      ls.win = true;
-      ls.win_known = known;
-      ls.win_base = known ? glo : 0;
-      ls.win_slots = slots;
-    } else if (slots > 0) {
-      set_error("");  // no room for the window: the table as it is
-    }
+    ls.win = slots > 0;
+    ls.win_known = known;
+    ls.win_base = known ? glo : 0;
+    ls.win_slots = slots;
   }
   // the room the launch policy plans with: the table's limit less the
   // reservations threads may hold unused
@@ -1488,8 +1489,7 @@ static wg_status run_device(const PipelineRun& r) {
     race = (int64_t)ls.grid * (ls.tile ? 32 * (1 + ls.cfg.consumers) : ls.block);
     if (bound + race > limit() && !a->spill) {  // a table that holds them, when it is small
       const int64_t nb = (int64_t)table_words(a, cap_for(bound + race)) * 8;
-      const int64_t budget = ctx->ledger.budget();
-      if (nb <= kSnapshotMaxBytes && (budget <= 0 || 2 * nb <= budget - ctx->ledger.used())) {
+      if (nb <= kSnapshotMaxBytes && 2 * nb <= hbm_room(ctx)) {
         WG_TRY(rebuild_table(a, cap_for(bound + race), a->L));
         WG_TRY(refresh_groups(a));
       }
@@ -1513,8 +1513,7 @@ static wg_status run_device(const PipelineRun& r) {
   if (!a->spill) {
     const int64_t want = std::max<int64_t>(a->hint, a->known_groups) + (int64_t)ls.grid * ls.block;
     const int64_t nb = (int64_t)table_words(a, cap_for(want)) * 8;
-    const int64_t budget = ctx->ledger.budget();
-    if (limit() < want && nb <= kSnapshotMaxBytes && (budget <= 0 || 2 * nb <= budget - ctx->ledger.used())) {
+    if (limit() < want && nb <= kSnapshotMaxBytes && 2 * nb <= hbm_room(ctx)) {
       WG_TRY(rebuild_table(a, cap_for(want), a->L));
       WG_TRY(refresh_groups(a));
     }
@@ -1709,8 +1708,7 @@ static bool hc_eligible(const PipelineRun& r, const wgd::Plan& P) {
   int64_t row_bytes = 0;
   for (int j = 0; j < P.n_in; ++j) row_bytes += wgd::cls_bytes(P.in[j].cls);
   const int64_t need = 2 * P.n_items * row_bytes + std::max<int64_t>(a->hint, 1024) * words * 8 * 5 / 4;
-  const Ledger& L = a->ctx->ledger;
-  return L.budget() <= 0 || L.budget() - L.used() >= need;
+  return hbm_room(a->ctx) >= need;
 }
 
 // The copy's column j as a plan input: class and element size from the plan
@@ -2211,7 +2209,7 @@ static wg_status spill_consume(const PipelineRun& r, const wgd::Plan& P0in, cons
   // windows of up to 2^24 rows, or what a quarter of the ledger's room holds
   int64_t row_bytes = 0;
   for (int e : a->sp_es) row_bytes += e;
-  const int64_t room = ctx->ledger.budget() > 0 ? ctx->ledger.budget() - ctx->ledger.used() : (int64_t(1) << 40);
+  const int64_t room = hbm_room(ctx);
   const int64_t n = P0.n_items;
   for (int j = 0; j < P0.n_in; ++j) row_bytes += a->sp_null[(size_t)j] ? 4 : 0;
   const int64_t win = std::max<int64_t>(int64_t(1) << 16, std::min<int64_t>(int64_t(1) << 24, room / 4 / std::max<int64_t>(row_bytes, 1))) &
@@ -2565,13 +2563,12 @@ Ctx* agg_ctx(wg_agg* a) { return a->ctx; }
 // Frees what an aggregate keeps only to speed up its next query (the
 // reordered input copy and its counters), for an aggregate parked in a pool.
 void agg_trim(wg_agg* a) {
-  if (a->part_bufs.empty() && !a->part_counts.get() && !a->win_buf.get()) return;
+  if (a->part_bufs.empty() && !a->part_counts.get()) return;
   ensure_device(a->ctx);
   cudaStreamSynchronize(a->ctx->stream);  // no launch still reads them
   a->part_bufs.clear();
   a->part_counts.reset();
   a->part_offs.reset();
-  a->win_buf.reset();
 }
 std::vector<int32_t> agg_input_cols(wg_agg* a) {
   std::vector<int32_t> r = a->key_cols;

@@ -135,28 +135,33 @@ wg_status send_pieces(Ctx* ctx, const std::vector<HostPiece>& pieces, int64_t by
 }
 
 // ---- parked blocks ---------------------------------------------------------
-// Device blocks of finished decodes, for the next one: a cudaMalloc and a
-// cudaFree of tens of megabytes cost milliseconds each on a device that holds
-// other large allocations (40 of them 18 and 21 ms of a 2^21-row scan).
-// At most kParkBytes per context and a sixteenth of its budget; outside the
-// ledger while parked (in it again once taken); dropped when the device runs
-// out of memory and with the context.
+// Device blocks of finished calls (decodes, key windows), for the next one: a
+// cudaMalloc and a cudaFree of tens of megabytes cost milliseconds each on a
+// device that holds other large allocations (40 of them 18 and 21 ms of a 2^21-row
+// scan). At most kParkBytes per context. A block is in one place at a time: taken,
+// it belongs to its taker alone; parked, to the list under its lock.
 constexpr int64_t kParkBytes = int64_t(256) << 20;
 
 wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out) {
+  const int64_t want = (bytes + 255) & ~int64_t(255);
   {
-    std::lock_guard<std::mutex> g(ctx->park_mu);
-    size_t best = ctx->parked.size();
-    for (size_t i = 0; i < ctx->parked.size(); ++i)
-      if (ctx->parked[i].bytes >= bytes && ctx->parked[i].bytes <= 2 * bytes + (int64_t(1) << 20) &&
-          (best == ctx->parked.size() || ctx->parked[i].bytes < ctx->parked[best].bytes))
+    std::lock_guard<std::mutex> g(ctx->park->mu);
+    auto& blocks = ctx->park->blocks;
+    // a little larger serves too (pages of one file differ in size); the taker is charged what it asked for
+    const int64_t most = want + std::max<int64_t>(want / 8, int64_t(1) << 20);
+    size_t best = blocks.size();
+    for (size_t i = 0; i < blocks.size(); ++i)
+      if (blocks[i].owner == ctx && blocks[i].bytes >= want && blocks[i].bytes <= most &&
+          (best == blocks.size() || blocks[i].bytes < blocks[best].bytes))
         best = i;
-    if (best < ctx->parked.size() && ctx->ledger.reserve(ctx->parked[best].bytes)) {
+    if (best < blocks.size()) {
       out->reset();
       out->ctx_ = ctx;
-      out->ptr_ = ctx->parked[best].ptr;
-      out->bytes_ = ctx->parked[best].bytes;
-      ctx->parked.erase(ctx->parked.begin() + (int64_t)best);
+      out->ptr_ = blocks[best].ptr;
+      out->bytes_ = want;
+      out->extra_ = blocks[best].bytes - want;
+      ctx->ledger.release(out->extra_);
+      blocks.erase(blocks.begin() + (int64_t)best);
       return WG_OK;
     }
   }
@@ -165,57 +170,58 @@ wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out) {
 
 void park_block(Ctx* ctx, DevBuf* b) {
   if (!b->ptr_) return;
-  const int64_t most = std::min<int64_t>(kParkBytes, ctx->ledger.budget() > 0 ? ctx->ledger.budget() / 16 : kParkBytes);
-  std::lock_guard<std::mutex> g(ctx->park_mu);
-  int64_t held = b->bytes_;
-  for (const auto& p : ctx->parked) held += p.bytes;
-  while (held > most && !ctx->parked.empty()) {  // the oldest go first
-    held -= ctx->parked.front().bytes;
-    cudaFree(ctx->parked.front().ptr);
-    ctx->parked.erase(ctx->parked.begin());
+  const int64_t size = b->bytes_ + b->extra_;
+  std::lock_guard<std::mutex> g(ctx->park->mu);
+  auto& blocks = ctx->park->blocks;
+  int64_t held = size;
+  for (const auto& p : blocks) held += p.owner == ctx ? p.bytes : 0;
+  for (size_t i = 0; size <= kParkBytes && held > kParkBytes && i < blocks.size();) {  // its oldest go first
+    if (blocks[i].owner != ctx) { ++i; continue; }
+    held -= blocks[i].bytes;
+    cudaFree(blocks[i].ptr);
+    ctx->ledger.release(blocks[i].bytes);
+    blocks.erase(blocks.begin() + (int64_t)i);
   }
-  if (held > most) {
+  if (held > kParkBytes || (b->extra_ > 0 && !ctx->ledger.reserve(b->extra_))) {
     b->reset();
     return;
   }
-  ctx->parked.push_back({b->ptr_, b->bytes_});
-  ctx->ledger.release(b->bytes_);
+  blocks.push_back({b->ptr_, size, ctx});
   b->ctx_ = nullptr;
   b->ptr_ = nullptr;
-  b->bytes_ = 0;
+  b->bytes_ = b->extra_ = 0;
 }
 
-bool drop_parked(Ctx* ctx) {
-  std::lock_guard<std::mutex> g(ctx->park_mu);
-  const bool any = !ctx->parked.empty();
-  for (const auto& p : ctx->parked) cudaFree(p.ptr);
-  ctx->parked.clear();
-  return any;
-}
-
-bool drop_spares(Ctx* ctx) {
-  std::lock_guard<std::mutex> g(ctx->spare_mu);
-  bool any = false;
-  for (SpareBuf* b : ctx->spares) {
-    any = any || b->get() != nullptr;
-    b->reset();  // (cudaFree waits for queued work)
+// Frees the parked blocks of the contexts that share ctx's list (only's alone,
+// when given). cudaFree waits for the work queued on them.
+static void free_parked(Park* park, const Ctx* only) {
+  std::lock_guard<std::mutex> g(park->mu);
+  size_t kept = 0;
+  for (const auto& p : park->blocks) {
+    if (only && p.owner != only) {
+      park->blocks[kept++] = p;
+      continue;
+    }
+    cudaFree(p.ptr);
+    p.owner->ledger.release(p.bytes);
   }
-  return any;
+  park->blocks.resize(kept);
 }
 
-wg_status SpareBuf::ensure(Ctx* ctx, int64_t bytes) {
-  if (listed_ == nullptr) {
-    std::lock_guard<std::mutex> g(ctx->spare_mu);
-    ctx->spares.push_back(this);
-    listed_ = ctx;
-  }
-  return DevBuf::ensure(ctx, bytes);
+void drop_parked(Ctx* ctx) { free_parked(ctx->park.get(), nullptr); }
+
+bool reserve_hbm(Ctx* ctx, int64_t bytes) {
+  if (ctx->ledger.reserve(bytes)) return true;
+  drop_parked(ctx);  // (or another thread has: its lock was waited for)
+  return ctx->ledger.reserve(bytes);
 }
 
-SpareBuf::~SpareBuf() {
-  if (!listed_) return;
-  std::lock_guard<std::mutex> g(listed_->spare_mu);
-  listed_->spares.erase(std::find(listed_->spares.begin(), listed_->spares.end(), this));
+int64_t hbm_room(Ctx* ctx) {
+  if (ctx->ledger.budget() <= 0) return int64_t(1) << 40;
+  std::lock_guard<std::mutex> g(ctx->park->mu);
+  int64_t room = ctx->ledger.budget() - ctx->ledger.used();
+  for (const auto& p : ctx->park->blocks) room += p.owner == ctx ? p.bytes : 0;
+  return room;
 }
 
 thread_local std::string t_err;
@@ -237,18 +243,16 @@ wg_status DevBuf::alloc(Ctx* ctx, int64_t bytes) {
   reset();
   if (bytes <= 0) return WG_OK;
   int64_t rounded = (bytes + 255) & ~int64_t(255);
-  if (!ctx->ledger.reserve(rounded) && !(drop_spares(ctx) && ctx->ledger.reserve(rounded)))
+  if (!reserve_hbm(ctx, rounded))
     return fail(WG_E_NOMEM, "HBM ledger: memory budget exceeded (used=" + std::to_string(ctx->ledger.used()) +
                                 ", requested=" + std::to_string(rounded) +
                                 ", budget=" + std::to_string(ctx->ledger.budget()) + ")");
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, (size_t)rounded);
   if (e == cudaErrorMemoryAllocation) {
-    const bool parked = drop_parked(ctx);
-    if (drop_spares(ctx) || parked) {
-      cudaGetLastError();
-      e = cudaMalloc(&p, (size_t)rounded);
-    }
+    cudaGetLastError();
+    drop_parked(ctx);
+    e = cudaMalloc(&p, (size_t)rounded);
   }
   if (e != cudaSuccess) {
     ctx->ledger.release(rounded);
@@ -270,7 +274,7 @@ void DevBuf::reset() {
     cudaFree(ptr_);
     ctx_->ledger.release(bytes_);
   }
-  ctx_ = nullptr; ptr_ = nullptr; bytes_ = 0;
+  ctx_ = nullptr; ptr_ = nullptr; bytes_ = 0; extra_ = 0;
 }
 
 int64_t elem_size(int32_t t) {
@@ -431,7 +435,9 @@ wg_status wg_ctx_create_child(wg_ctx* parent, wg_ctx** out) {
   if (!parent || !out) return fail(WG_E_INVALID, "NULL argument");
   *out = nullptr;
   WG_TRY(ensure_device(parent));
-  return ctx_make(parent->device, parent->ledger.budget(), &parent->ledger, parent->pinned_spill_bytes, out);
+  WG_TRY(ctx_make(parent->device, parent->ledger.budget(), &parent->ledger, parent->pinned_spill_bytes, out));
+  (*out)->park = parent->park;
+  return WG_OK;
 }
 
 wg_status wg_ctx_destroy(wg_ctx* c) {
@@ -445,7 +451,7 @@ wg_status wg_ctx_destroy(wg_ctx* c) {
     if (c->h2d_done[i]) cudaEventDestroy(c->h2d_done[i]);
     c->win[i].reset();
   }
-  drop_parked(c);
+  free_parked(c->park.get(), c);
   if (c->pinned) cudaFreeHost(c->pinned);
   if (c->out_pinned) cudaFreeHost(c->out_pinned);
   for (cudaEvent_t e : c->out_ev)
@@ -476,7 +482,7 @@ wg_status wg_ledger_stats(wg_ctx* c, int64_t* used, int64_t* peak, int64_t* budg
 
 wg_status wg_ledger_reserve(wg_ctx* c, int64_t bytes) {
   if (!c || bytes < 0) return fail(WG_E_INVALID, "bad ledger reservation");
-  if (!c->ledger.reserve(bytes) && !(drop_spares(c) && c->ledger.reserve(bytes))) return fail(WG_E_NOMEM, "HBM ledger: memory budget exceeded");
+  if (!reserve_hbm(c, bytes)) return fail(WG_E_NOMEM, "HBM ledger: memory budget exceeded");
   return WG_OK;
 }
 

@@ -8,6 +8,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -86,8 +87,8 @@ class DevBuf {
   DevBuf& operator=(DevBuf&& o) noexcept {
     if (this != &o) {
       reset();
-      ctx_ = o.ctx_; ptr_ = o.ptr_; bytes_ = o.bytes_;
-      o.ctx_ = nullptr; o.ptr_ = nullptr; o.bytes_ = 0;
+      ctx_ = o.ctx_; ptr_ = o.ptr_; bytes_ = o.bytes_; extra_ = o.extra_;
+      o.ctx_ = nullptr; o.ptr_ = nullptr; o.bytes_ = 0; o.extra_ = 0;
     }
     return *this;
   }
@@ -105,21 +106,21 @@ class DevBuf {
   Ctx* ctx_ = nullptr;
   void* ptr_ = nullptr;
   int64_t bytes_ = 0;
+  int64_t extra_ = 0;  // a taken block's bytes beyond what was asked for (not charged)
 };
 
-// A buffer kept between calls that its owner can do without (it checks get()
-// before each use): dropped when the ledger would refuse an allocation of its
-// context, so keeping it refuses nothing that ran without it.
-class SpareBuf : public DevBuf {
- public:
-  SpareBuf() = default;
-  SpareBuf(const SpareBuf&) = delete;
-  SpareBuf& operator=(const SpareBuf&) = delete;
-  ~SpareBuf();
-  wg_status ensure(Ctx* ctx, int64_t bytes);
-
- private:
-  Ctx* listed_ = nullptr;
+// Device blocks that no call uses, kept for the next one that needs their size
+// (take_block / park_block), of a context and its children. Each is charged to
+// its owner's ledger and given back when a reservation of any of these contexts
+// would be refused, so keeping it refuses nothing.
+struct Park {
+  struct Block {
+    void* ptr;
+    int64_t bytes;
+    Ctx* owner;
+  };
+  std::mutex mu;
+  std::vector<Block> blocks;  // oldest first
 };
 
 // ---- context ---------------------------------------------------------------
@@ -155,15 +156,7 @@ struct Ctx {
   char* out_pinned = nullptr;
   cudaEvent_t out_ev[2] = {nullptr, nullptr};
   std::mutex out_mu;
-  // device blocks kept for reuse (take_block / park_block)
-  struct Parked {
-    void* ptr;
-    int64_t bytes;
-  };
-  std::vector<Parked> parked;
-  std::mutex park_mu;
-  std::vector<SpareBuf*> spares;  // of the context's objects
-  std::mutex spare_mu;
+  std::shared_ptr<Park> park = std::make_shared<Park>();  // a child shares its parent's
 
   explicit Ctx(int64_t budget, Ledger* parent = nullptr) : ledger(budget, parent) {}
   void count_launch(int n = 1) { launches.fetch_add(n); }
@@ -185,12 +178,16 @@ struct HostPiece {
 wg_status send_pieces(Ctx* ctx, const std::vector<HostPiece>& pieces, int64_t bytes, char* dst);
 
 // A device block of at least `bytes` for a buffer that the context's stream
-// alone uses, charged to the ledger: a parked one that fits, else a new one.
-// park_block gives it back once no queued work on any stream uses it.
+// alone uses, charged to the ledger: a parked one that fits, else a new one. It is
+// the caller's alone until park_block gives it back, once every use of it is
+// queued on the context's stream (the next taker's work follows there) or done.
 wg_status take_block(Ctx* ctx, int64_t bytes, DevBuf* out);
 void park_block(Ctx* ctx, DevBuf* b);
-bool drop_parked(Ctx* ctx);
-bool drop_spares(Ctx* ctx);  // whether any held memory
+void drop_parked(Ctx* ctx);
+// A ledger reservation, for which parked blocks give way.
+bool reserve_hbm(Ctx* ctx, int64_t bytes);
+// What the context's budget has left, parked blocks included (no budget: 2^40).
+int64_t hbm_room(Ctx* ctx);
 
 wg_status ensure_device(Ctx* ctx);           // cudaSetDevice(ctx->device)
 wg_status read_back_i64(Ctx* ctx, const int64_t* dev, int64_t* out, int n);

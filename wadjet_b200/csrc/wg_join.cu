@@ -639,7 +639,7 @@ static wg_status grace_plan(wg_join* j) {
   // and the direct table (at most 4 slots of 8 bytes), and each payload column
   int64_t row_bytes = j->key.es + 4 + 64 + 32;
   for (const BuildCol& c : j->pay) row_bytes += c.es + 1;
-  const int64_t left = ctx->ledger.budget() - ctx->ledger.used();
+  const int64_t left = hbm_room(ctx);
   const int64_t room = std::max<int64_t>(left / 2, 1 << 20);
   j->passes.clear();
   const int np = (int)j->parts.size();

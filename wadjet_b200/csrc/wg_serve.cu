@@ -144,7 +144,7 @@ void worker_main(wg_server* s, int slot_idx) {
           // admission: the device has room for more work (or is idle), and the
           // head request's footprint fits the shared ledger
           const bool room = s->running == 0 || s->inflight_work + head->work <= s->work_limit;
-          if (room && s->ctx->ledger.reserve(head->est)) {
+          if (room && reserve_hbm(s->ctx, head->est)) {
             head->held = true;
             s->queue.pop_front();
             r = head;
