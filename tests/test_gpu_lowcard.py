@@ -164,3 +164,40 @@ def test_row_counters_of_a_skewed_join_key(ctx, monkeypatch):
     monkeypatch.setenv("WG_AGG_SMEM", "0")
     assert_groups_equal(got, run(), ["sum_i", "count"])
     join.close()
+
+
+@pytest.mark.parametrize("jtype", [None, "left"])
+@pytest.mark.parametrize("packed", [False, True])
+@pytest.mark.parametrize("groups", [900, 30_000])
+def test_groups_far_beyond_the_hint(ctx, monkeypatch, packed, groups, jtype):
+    """Hints 10 to 10,000 times too low: rows without a slot, the second layout, the rows that
+    find none there either, and chained join matches among them."""
+    import wadjet_b200 as wg
+    n = 300_007
+    rng = np.random.default_rng(groups + packed)
+    key = rng.integers(0, groups // (10 if packed else 1), n) * 1_000_003
+    key[:50] = EMPTY
+    cols = [wg.Column(I64, key, rng.random(n) >= 0.01), wg.Column(I32, rng.integers(0, 10, n, dtype=np.int32)),
+            wg.Column(F64, rng.random(n), rng.random(n) >= 0.1), wg.Column(I64, rng.integers(-(1 << 40), 1 << 40, n)),
+            wg.Column(I64, rng.integers(0, 600, n) * 7)]
+    join, kw = None, {}
+    if jtype:
+        join = wg.HashJoin(ctx, 0, 4, payload=[1], build_row_hint=1200, join_type=wg.abi.JOIN_LEFT)
+        join.build([wg.Batch([wg.Column(I64, np.arange(1000) % 400 * 7), wg.Column(I32, np.arange(1000, dtype=np.int32))])])
+        kw["join"] = join
+    aggs = [wg.AggColumn(wg.AGG_SUM, 2), wg.AggColumn(wg.AGG_SUM, 3), wg.AggColumn(wg.AGG_MAX, 3),
+            wg.AggColumn(wg.AGG_COUNT, 5 if jtype else 2)]
+    for hint in (3, 90, 900):
+        def run():
+            a = wg.HashAggregate(ctx, [0, 1] if packed else [0], aggs, ndv_hint=hint)
+            wg.run_pipeline(ctx, wg.Batch(cols), a, filters=[(1, wg.OP_LT, 9)], **kw)
+            a.finalize()
+            e = a.export()
+            a.close()
+            return e
+        monkeypatch.setenv("WG_AGG_SMEM", "1")
+        got = run()
+        monkeypatch.setenv("WG_AGG_SMEM", "0")
+        assert_groups_equal(got, run(), ["sum_f", "sum_i", "max_i", "count"], rel=1e-11)
+    if join:
+        join.close()

@@ -1123,7 +1123,7 @@ static int64_t smem_rows_per_cta(int64_t n, int64_t groups) {
 static void leave_shared(const Ctx* ctx, LaunchSpec& ls, bool stat, int blocks_per_sm) {
   ls.smem = ls.lc = ls.stage = false;
   ls.smem_bytes = 0;
-  ls.P.smem_slots = 0;
+  ls.P.smem_slots = ls.P.smem_more = 0;
   ls.P.gdense = 0;
   if (ls.tile) return;
   const int64_t n = ls.P.n_items;
@@ -1168,6 +1168,9 @@ static void lowcard_setup(wg_agg* a, LaunchSpec& ls, int64_t expect, bool ranged
     ls.P.smem_slots = (int32_t)S;
     ls.P.smem_sw = (int32_t)aw;
     ls.P.smem_rep = R;
+    // the same bytes as slots of one copy, for a CTA that meets more groups
+    const int64_t more = kw > 0 && !dense && R > 1 ? (S * key_bytes + (R * (S + 2) - 2) * aw * 8) / (key_bytes + aw * 8) : 0;
+    ls.P.smem_more = (int32_t)std::min<int64_t>(more, 16384);
     ls.P.gdense = dense ? 1 : 0;
     ls.P.gmin = glo;
     ls.smem_bytes = (size_t)(S * key_bytes + R * (S + 2) * aw * 8);

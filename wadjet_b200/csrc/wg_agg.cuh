@@ -95,6 +95,7 @@ struct Plan {
   int32_t n_in, n_filters, has_join, n_exprs;
   int32_t probe_col;
   int32_t smem_slots;            // >0: CTA-private shared-memory table of this many slots
+  int32_t smem_more;             // slots of one copy in the same bytes, 0: no such layout (lowcard_kernel)
   int32_t shape;                 // compiled query shape (wg_shapes.cuh), 0 = generic
   int32_t prefetch;              // grid-stride iterations of input prefetched into L2 ahead (0 = off)
   int32_t smem_sw;               // words per shared-table slot (0 = the layout's slot_words)

@@ -153,6 +153,7 @@ struct DynShape {
 template <class C>
 struct StatShape {
   static constexpr bool smem_ok = C::smem_ok;
+  static constexpr int kAggs = C::n_aggs;
   // straight-line code fits 40 registers: two 768-thread CTAs per SM (48 warps)
   static constexpr int kBlock = 768, kMinBlocks = 2;
   // vector kernel: evaluate all of a lane's rows before their table updates

@@ -5,7 +5,7 @@
 // groups, float-SUM copies, warp combine, HBM-table rows), deciding per row
 // from the plan: 234 warp instructions per 32 rows of the group-by shape, whose
 // shared-memory work is five operations, so it was bound by instruction issue
-// (1969 us at 2^28 rows, 4096 groups; 1570 here; the columns take 1149 us at the
+// (1969 us at 2^28 rows, 4096 groups; 1405 here; the columns take 1149 us at the
 // copy peak). Here a row is its loads, the comparison, a 32-bit multiply-shift hash,
 // one key read and its updates; the first probes of a lane's rows are read
 // together. Float SUMs accumulate in scaled fixed point (f64_to_fixed_scaled)
@@ -17,7 +17,10 @@
 // around them. (4096 keys hashed into 5760 slots take 2.2 probes on average.)
 //
 // A row whose key finds no slot (outside the window, the table at its fill limit,
-// the key equal to the empty pattern) goes to the HBM table.
+// no free slot within kLeanProbes steps, the key equal to the empty pattern) goes to
+// the HBM table, 32 of a warp's at a time, by the shape's own code. (2^24 rows into 3000
+// sparse keys with a hint of 300, a sixth of them without a slot: 1.95 ms a row at a time and
+// interpreted, 0.54 so.)
 #pragma once
 
 #include "wg_lowcard.cuh"
@@ -25,9 +28,11 @@
 namespace wgd {
 
 // Rows per lane and an L2 prefetch two chunks ahead, group-by shape at 2^28 rows
-// and 4096 groups: 4 without 1570, 2 without 1673, 4 with 1832, 2 with 1831 us;
-// the next chunk's loads held in registers (spills) 2962 with 4 and 3141 with 2.
+// and 4096 groups (with rows for the HBM table handled in the loop, 1570 us as it was then): 4
+// without 1570, 2 without 1673, 4 with 1832, 2 with 1831 us; the next chunk's loads held
+// in registers (spills) 2962 with 4 and 3141 with 2.
 constexpr int kLeanRows = 4;
+constexpr int kLeanProbes = 16;    // slots a key is looked for in (two in a thousand keys of a table 3/4 full need more)
 constexpr int kLeanThreads = 1024; // per SM (64 registers each), in one CTA or two
 
 template <class C>
@@ -42,39 +47,42 @@ constexpr int lean_stride(bool fixed) {
   return (C::slot_words + (fixed ? 2 * lean_float_sums<C>() : 0)) | 1;
 }
 
-// Insert or find from slot h on: the slot's index, -1 when the table has no room for the key.
-// A thread reserves its place in *s_groups before it installs a key and gives it back when
-// another thread's key took the slot, so the table never holds more than s_limit < S keys: with
-// a check before and an add after, every thread between the two passes the limit, and a small
-// table (256 slots, 32 of them spare) fills.
+// A thread's place among s_limit, held before it installs a key, so that the table never
+// holds more: with a check before and an add after, every thread between the two passed
+// the limit, and a small table (256 slots, 32 of them spare) filled.
+__device__ __forceinline__ bool reserve_group(int* s_groups, int s_limit) {
+  if (*((volatile int*)s_groups) >= s_limit) return false;
+  if (atomicAdd(s_groups, 1) < s_limit) return true;
+  atomicSub(s_groups, 1);
+  return false;
+}
+
+// The stride of a key's probes: its own, so that a table near its limit has no long runs.
+__device__ __forceinline__ uint32_t lean_step(unsigned long long k) {
+  return 1u + ((uint32_t)((k * 0x9E3779B97F4A7C15ULL) >> 32) & 31u);
+}
+
+// Insert or find from slot h on within `probes` slots: the slot's index, -1 when the key has none.
 template <int SW>
-static __device__ __noinline__ int lean_insert(unsigned long long* sm, int S, unsigned long long k, uint32_t h, int* s_groups,
-                                        int s_limit) {
+static __device__ __noinline__ int lean_insert(unsigned long long* sm, int S, unsigned long long k, uint32_t h, int probes,
+                                               int* s_groups, int s_limit) {
   if (k == WG_EMPTY_KEY) return -1;
-  for (int p = 0; p < S; ++p) {
+  const uint32_t step = lean_step(k);
+  for (; probes > 0; --probes) {
     unsigned long long* s = sm + h * SW;
     const unsigned long long cur = *((volatile unsigned long long*)s);
     if (cur == k) return (int)h;
     if (cur == WG_EMPTY_KEY) {
-      if (*((volatile int*)s_groups) >= s_limit) return -1;
-      if (atomicAdd(s_groups, 1) >= s_limit) {
-        atomicSub(s_groups, 1);
-        return -1;
-      }
+      if (!reserve_group(s_groups, s_limit)) return -1;
       const unsigned long long old = atomicCAS(s, WG_EMPTY_KEY, k);
       if (old == WG_EMPTY_KEY) return (int)h;
       atomicSub(s_groups, 1);
       if (old == k) return (int)h;
     }
-    h = h + 1 == (uint32_t)S ? 0u : h + 1;
+    h += step;
+    if (h >= (uint32_t)S) h -= (uint32_t)S;
   }
   return -1;
-}
-
-// The rows r0 + u of the bits u of `far`, into the HBM table.
-static __device__ __noinline__ void lean_far_rows(const Plan& P, int64_t r0, unsigned far, Credit* cr) {
-#pragma unroll 1
-  for (; far; far &= far - 1) lc_far_row(P, r0 + __ffs(far) - 1, -1, cr);
 }
 
 // What a CTA takes from its sample of the input.
@@ -125,6 +133,8 @@ __device__ __forceinline__ void lean_rows(const Plan& P, int64_t begin, int64_t 
   const int lane = threadIdx.x & 31;
   const int s_limit = (S * 7) / 8;
   int64_t base = begin + first * (32 * U);
+  FarQueue queue;
+  far_init(queue, base);
   for (;;) {
     // the common rows; a chunk with rows for the HBM table leaves the loop, so
     // that the call below holds no registers through it
@@ -169,12 +179,17 @@ __device__ __forceinline__ void lean_rows(const Plan& P, int64_t begin, int64_t 
         int at = (int)h[u];
         if (!DENSE) {
           unsigned long long c = cur[u];
-          while (c != k && c != WG_EMPTY_KEY) {  // at most once around the table
-            at = at + 1 == S ? 0 : at + 1;
-            if (at == (int)h[u]) break;
-            c = *((volatile unsigned long long*)(sm + at * SW));
+          int probes = kLeanProbes;
+          if (c != k && c != WG_EMPTY_KEY) {
+            const int step = (int)lean_step(k);
+            do {
+              at += step;
+              if (at >= S) at -= S;
+              c = *((volatile unsigned long long*)(sm + at * SW));
+            } while (c != k && c != WG_EMPTY_KEY && --probes > 0);
           }
-          if (c == WG_EMPTY_KEY) at = lean_insert<SW>(sm, S, k, (uint32_t)at, s_groups, s_limit);
+          if (c == WG_EMPTY_KEY && *((volatile int*)s_groups) >= s_limit) at = -1;
+          else if (c == WG_EMPTY_KEY) at = lean_insert<SW>(sm, S, k, (uint32_t)at, probes, s_groups, s_limit);
           else if (c != k) at = -1;
           if (at < 0) { far |= 1u << u; continue; }
         }
@@ -184,10 +199,11 @@ __device__ __forceinline__ void lean_rows(const Plan& P, int64_t begin, int64_t 
       }
       if (__any_sync(WG_FULL_MASK, far != 0)) break;
     }
-    if (base >= end) return;
-    if (far) lean_far_rows(P, base + (int64_t)lane * U, far, cr);
+    if (base >= end) break;
+    far_rows<StatShape<C>, U, false>(P, &queue, far, cr, base + (int64_t)lane * U);
     base += step * (32 * U);
   }
+  far_flush<StatShape<C>>(P, &queue, cr);
 }
 
 // One row per thread, spread over [begin, end) so that neither order nor a

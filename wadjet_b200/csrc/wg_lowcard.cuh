@@ -18,22 +18,33 @@
 //    As many copies as fit the CTA's share of shared memory are taken; the
 //    flush folds them with shuffles and updates the HBM table once per group.
 //
+// The copies are for the groups that the caller expects, and an estimate may be ten
+// times too low. Where many of a CTA's rows found no slot, it hands its groups to the
+// HBM table and goes on with as many slots of one copy as its shared memory holds
+// (lc_rest, apart from the common loop, whose registers it would take). 2^24 rows into
+// 1000 groups with a hint of 100: 36.6 ms with probes as long as the full table and
+// a row at a time into the HBM table, 0.54 now, 0.33 with the right hint; into 10,000 by
+// two keys with a hint of 1000 35.3 and 2.3 ms.
+//
 // Packed keys, NULL keys, a scalar aggregate (no key) and NULL counters take
-// this path too. Rows whose key finds no slot (the key table at its fill limit, a key
-// outside a dense range) go to the HBM table as in pipeline_kernel, the path
-// of plans whose groups do not fit.
+// this path too. Rows whose key finds no slot (none free within kLcProbes, or a key
+// outside a dense range) go to the HBM table, 32 of a warp's at a time; a warp that
+// still meets many such rows stops looking for slots.
 //
 // Measured on B200, against pipeline_kernel: 30,000,001 rows, 6 groups by two
 // int32 keys, seven aggregates over nullable columns 14.74 -> 1.58 ms (both
 // bound by instruction issue and its latencies, not by the 1.33 GB read); a LEFT
 // join of 2^24 + 3 rows on sparse int64 keys with duplicates, 50 groups 4.37 ->
-// 0.89 ms. Rows per lane x threads per SM, the first query: 2 x 1024 1.58, 3 x
+// 0.89 ms. Shared memory beyond the tables' need costs: 64 KB more of it per CTA left so
+// little L1 that the first query took 2.3 ms. Rows per lane x threads per SM, the first query: 2 x 1024 1.58, 3 x
 // 1024 1.50, 4 x 768 1.66, 2 x 768 1.81, 4 x 512 1.85, 2 x 1536 1.86 ms; the second
 // 0.89, 0.88, 0.96, 1.05, 1.06, 0.87; 2^21 rows into 1000 groups 93, 104, 110, 103,
 // 104, 106 us.
 #pragma once
 
 #include "wg_shapes.cuh"
+
+#include <type_traits>
 
 namespace wgd {
 
@@ -290,36 +301,40 @@ __device__ __forceinline__ void lc_value(const Plan& P, const LcRowSet& r, const
   }
 }
 
-// A key's slot in the CTA's key table, inserting it: [0, S) a regular key, S
-// the key equal to the empty pattern, S + 1 the NULL key; -1 when the table is
-// at its fill limit or the key outside a dense range (or, with the groups in a
-// key window in HBM, outside the window or NULL).
+// Slots a key is looked for in before it counts as having none: probes of a full
+// table are instructions of every row. (Keys at half load do not need so many, also where small
+// packed keys hash to neighbouring slots.)
+constexpr int kLcProbes = 32;
+
+// A key's slot in the CTA's key table of S slots, inserting it: [0, S) a regular
+// key, S the key equal to the empty pattern, S + 1 the NULL key; -1 when it has
+// none or is outside a dense range (or, with the groups in a key window in HBM,
+// outside the window or NULL).
 template <bool SH>
-__device__ __forceinline__ int lc_slot(const Plan& P, const KeyWindow& w, unsigned long long* keys, unsigned long long k0,
-                                       unsigned long long k1, bool knull, int* s_groups, int s_limit) {
+__device__ __forceinline__ int lc_slot(const Plan& P, const KeyWindow& w, unsigned long long* keys, int S,
+                                       unsigned long long k0, unsigned long long k1, bool knull) {
   if (!SH) {
     const unsigned long long d = k0 - (unsigned long long)w.base;
     return !knull && d < w.n ? (int)d : -1;
   }
-  const int S = P.smem_slots, kw = P.L.key_words;
+  const int kw = P.L.key_words;
   if (kw == 0) return 0;
   if (knull) return S + 1;
   if (P.gdense) {
     const uint32_t d = (uint32_t)k0 - (uint32_t)P.gmin;
     return d < (uint32_t)S ? (int)d : -1;
   }
+  const int probes = min(S, kLcProbes);
   if (kw == 1) {
     if (k0 == WG_EMPTY_KEY) return S;
     uint32_t h = __umulhi((uint32_t)((k0 * 0x9E3779B97F4A7C15ULL) >> 32), (uint32_t)S);
-    for (int p = 0; p < S; ++p) {
+    for (int p = 0; p < probes; ++p) {
       unsigned long long* s = keys + h;
       const unsigned long long cur = *((volatile unsigned long long*)s);
       if (cur == k0) return (int)h;
       if (cur == WG_EMPTY_KEY) {
-        if (*((volatile int*)s_groups) >= s_limit) return -1;
         const unsigned long long old = atomicCAS(s, WG_EMPTY_KEY, k0);
-        if (old == WG_EMPTY_KEY) { atomicAdd(s_groups, 1); return (int)h; }
-        if (old == k0) return (int)h;
+        if (old == WG_EMPTY_KEY || old == k0) return (int)h;
       }
       h = h + 1 == (uint32_t)S ? 0u : h + 1;
     }
@@ -328,7 +343,7 @@ __device__ __forceinline__ int lc_slot(const Plan& P, const KeyWindow& w, unsign
   if (k0 == ~0ULL && k1 == ~0ULL) return S;
   const unsigned long long m = (k0 ^ 0x9E3779B97F4A7C15ULL) * (k1 * 0x517CC1B727220A95ULL + 0x9E3779B97F4A7C15ULL | 1ULL);
   uint32_t h = __umulhi((uint32_t)(m >> 32), (uint32_t)S);
-  for (int p = 0; p < S; ++p) {
+  for (int p = 0; p < probes; ++p) {
     unsigned long long* s = keys + 2 * h;
     // the words change once, from {~0, ~0} to the key: a read with neither ~0
     // is the complete key, anything else is settled by the 16-byte CAS
@@ -338,9 +353,8 @@ __device__ __forceinline__ int lc_slot(const Plan& P, const KeyWindow& w, unsign
     } else {
       U128 e; e.lo = ~0ULL; e.hi = ~0ULL;
       U128 k; k.lo = k0; k.hi = k1;
-      if (*((volatile int*)s_groups) >= s_limit) return -1;
       const U128 old = cas128((U128*)s, e, k);
-      if (old.lo == e.lo && old.hi == e.hi) { atomicAdd(s_groups, 1); return (int)h; }
+      if (old.lo == e.lo && old.hi == e.hi) return (int)h;
       if (old.lo == k0 && old.hi == k1) return (int)h;
     }
     h = h + 1 == (uint32_t)S ? 0u : h + 1;
@@ -348,36 +362,17 @@ __device__ __forceinline__ int lc_slot(const Plan& P, const KeyWindow& w, unsign
   return -1;
 }
 
-// One row whose key found no shared slot, into the HBM table (rare: a hint far
-// below the groups there are). Neither inlined nor handed the key: it would hold
-// registers through every row's common path.
-static __device__ __noinline__ void lc_far_row(const Plan& P, int64_t row, int32_t brow, Credit* cr) {
-  const DynShape sh{P};
-  const SrcGlobal src{row};
-  ExprVals ev;
-  Contrib<WG_MAX_AGGS> c;
-  eval_exprs(P, sh, src, brow, ev);
-  unsigned long long k0, k1;
-  bool knull;
-  if (!make_key(P, sh, src, brow, ev, k0, k1, knull)) return;
-  make_contrib<WG_MAX_AGGS>(P, sh, src, brow, ev, c);
-  unsigned long long* g = find_global(sh, P.T, k0, k1, knull, P.err, cr);
-  if (g != nullptr) apply<WG_MAX_AGGS, false>(sh, g, c, 1ULL, 1, P.minmax_test != 0);
-}
-
-// Group keys of the rows in `live` and their shared slots; returns the rows
-// that have one, `far` the rows that have none.
-template <bool SH>
-__device__ __forceinline__ unsigned lc_keys(const Plan& P, const KeyWindow& w, const LcRowSet& r, const LcExprs& ev,
-                                            unsigned live, unsigned long long* keys, int (&slot)[kLcRows], unsigned& far, int* s_groups,
-                                            int s_limit) {
+// Group keys of the rows in `live`, packed as make_key does; returns the rows that have one.
+__device__ __forceinline__ unsigned lc_make_keys(const Plan& P, const LcRowSet& r, const LcExprs& ev, unsigned live,
+                                                 unsigned long long (&k0)[kLcRows], unsigned long long (&k1)[kLcRows],
+                                                 unsigned& knull) {
   const Layout& L = P.L;
-  unsigned long long k0[kLcRows], k1[kLcRows];
-  unsigned knull = 0, bad = 0;
-  WG_LC_EACH(u) { k0[u] = 0; k1[u] = 0; slot[u] = 0; }
+  unsigned bad = 0;
+  knull = 0;
+  WG_LC_EACH(u) { k0[u] = 0; k1[u] = 0; }
   if (L.key_words > 0) {
 #pragma unroll 1
-    for (int k = 0; k < L.n_keys; ++k) {  // make_key's packing
+    for (int k = 0; k < L.n_keys; ++k) {
       LcVals v;
       lc_value(P, r, ev, L.key_vcol[k], live, v);
       if (L.key_words == 1) {
@@ -399,11 +394,23 @@ __device__ __forceinline__ unsigned lc_keys(const Plan& P, const KeyWindow& w, c
       }
     }
     if (bad) set_error(P.err, WG_DERR_NULL_PACKED);
-    live &= ~bad;
   }
+  return live & ~bad;
+}
+
+// Group keys of the rows in `live` and their shared slots; returns the rows
+// that have one, `far` the rows that have none.
+template <bool SH>
+__device__ __forceinline__ unsigned lc_keys(const Plan& P, const KeyWindow& w, const LcRowSet& r, const LcExprs& ev,
+                                            unsigned live, unsigned long long* keys, int S, int (&slot)[kLcRows],
+                                            unsigned& far) {
+  unsigned long long k0[kLcRows], k1[kLcRows];
+  unsigned knull;
+  live = lc_make_keys(P, r, ev, live, k0, k1, knull);
+  WG_LC_EACH(u) slot[u] = 0;
   far = 0;
   WG_LC_LIVE(u, live) {
-    slot[u] = lc_slot<SH>(P, w, keys, k0[u], k1[u], (knull >> u) & 1u, s_groups, s_limit);
+    slot[u] = lc_slot<SH>(P, w, keys, S, k0[u], k1[u], (knull >> u) & 1u);
     far |= slot[u] < 0 ? 1u << u : 0u;
   }
   return live & ~far;
@@ -493,14 +500,141 @@ __device__ __forceinline__ void lc_update(const Plan& P, const LcRowSet& r, cons
   }
 }
 
-// The CTA's groups folded over their copies (R consecutive lanes per group) and
+// One row without a slot, into the HBM table: of a compiled shape row by row, of
+// any other plan by the same steps as the common rows'.
+template <class Sh>
+static __device__ __noinline__ void lc_far_row(const Plan& P, int64_t row, int32_t brow, Credit* cr) {
+  const Sh sh{P};
+  if constexpr (std::is_same<Sh, DynShape>::value) {
+    LcRowSet r;
+    r.base = row;
+    WG_LC_EACH(u) { r.off[u] = 0; r.brow[u] = brow; }
+    LcExprs ev;
+#pragma unroll 1
+    for (int e = 0; e < P.n_exprs; ++e) lc_eval(P, r, e, 1u, ev.v + e * kLcRows, ev.null[e]);
+    unsigned long long k0[kLcRows], k1[kLcRows];
+    unsigned knull;
+    if (!lc_make_keys(P, r, ev, 1u, k0, k1, knull)) return;
+    unsigned long long* g = find_global(sh, P.T, k0[0], k1[0], (knull & 1u) != 0, P.err, cr);
+    const int slot[kLcRows] = {0, 0};
+    if (g != nullptr) lc_update<false>(P, r, ev, 1u, g + P.L.key_words, slot);
+  } else {
+    constexpr int NA = Sh::kAggs;
+    const SrcGlobal src{row};
+    ExprVals ev;
+    Contrib<NA> c;
+    eval_exprs(P, sh, src, brow, ev);
+    unsigned long long k0, k1;
+    bool knull;
+    if (!make_key(P, sh, src, brow, ev, k0, k1, knull)) return;
+    make_contrib<NA>(P, sh, src, brow, ev, c);
+    unsigned long long* g = find_global(sh, P.T, k0, k1, knull, P.err, cr);
+    if (g != nullptr) apply<NA, false>(sh, g, c, 1ULL, 1, P.minmax_test != 0);
+  }
+}
+
+// The lane of the n-th set bit of m (n below its count).
+__device__ __forceinline__ int nth_lane(unsigned m, int n) {
+  int at = 0;
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) {
+    const int c = __popc(m & ((1u << s) - 1u));
+    if (n >= c) {
+      n -= c;
+      m >>= s;
+      at += s;
+    }
+  }
+  return at;
+}
+
+// Rows for the HBM table, gathered per warp until there are 32, one in each lane: a
+// row there is some hundreds of instructions and dependent reads, which cost a warp
+// the same for one row as for 32. In local memory, as it is used rarely: shared
+// memory taken for it would come out of the L1 cache, which the plan's steps use.
+struct FarQueue {
+  int64_t row;
+  int32_t brow;
+  int n;           // rows in the queue (all lanes the same, as are the fields below)
+  int far, mark;   // rows that came here since the last look, and how many the next one waits for
+  int64_t from;    // the row at which the warp began to count them
+};
+
+__device__ __forceinline__ void far_init(FarQueue& q, int64_t from) {
+  q.row = 0;
+  q.brow = -1;
+  q.n = q.far = 0;
+  q.mark = 64;
+  q.from = from;
+}
+
+template <class Sh>
+static __device__ __noinline__ void far_flush(const Plan& P, FarQueue* q, Credit* cr) {
+  if ((int)(threadIdx.x & 31) < q->n) lc_far_row<Sh>(P, q->row, q->brow, cr);
+  q->n = 0;
+  __syncwarp();
+}
+
+// Whether more than one in `share` of the warp's rows had no slot, looked at every q->mark such rows.
+static __device__ __noinline__ bool lc_too_many(FarQueue* q, int64_t base, int share) {
+  if (q->far < q->mark) return false;
+  const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * (32 * kLcRows);
+  const int64_t rows = ((base - q->from) / step + 1) * (32 * kLcRows);
+  const bool many = (int64_t)q->far * share > rows;
+  q->far = 0;
+  q->from = base + step;
+  return many;
+}
+
+// Every lane of the warp calls it: the rows row0 + u of the set bits u of `far`
+// (JOIN: two rows, row0 and row1, with their build rows). Returns lc_too_many, of
+// the rows up to base, where a share is given; one call for both, as every call in a
+// row loop costs the loop registers.
+template <class Sh, int U, bool JOIN>
+static __device__ __noinline__ bool far_rows(const Plan& P, FarQueue* q, unsigned far, Credit* cr, int64_t row0, int64_t row1 = 0,
+                                             int32_t b0 = -1, int32_t b1 = -1, int64_t base = 0, int share = 0) {
+  static_assert(!JOIN || U == 2, "two rows per lane with build rows");
+  const int lane = threadIdx.x & 31;
+  int n = q->n;
+#pragma unroll 1
+  for (int u = 0; u < U; ++u) {
+    const unsigned m = __ballot_sync(WG_FULL_MASK, (far >> u) & 1u);
+    if (m == 0) continue;
+    const int c = __popc(m);
+    const int64_t row = JOIN ? (u ? row1 : row0) : row0 + u;
+    const int32_t brow = u ? b1 : b0;
+    // row i of the step goes to lane n + i, past lane 31 to lane n + i - 32 once the queue has run
+    auto put = [&](int i) {
+      const bool in = i >= 0 && i < c;
+      const int from = in ? nth_lane(m, i) : lane;
+      const int64_t r = __shfl_sync(WG_FULL_MASK, row, from);
+      const int32_t b = JOIN ? __shfl_sync(WG_FULL_MASK, brow, from) : -1;
+      if (in) {
+        q->row = r;
+        q->brow = b;
+      }
+    };
+    put(lane - n);
+    if (n + c >= 32) {
+      lc_far_row<Sh>(P, q->row, q->brow, cr);
+      __syncwarp();
+      put(lane + 32 - n);
+    }
+    n = (n + c) & 31;
+    q->far += c;
+  }
+  q->n = n;
+  return share > 0 && lc_too_many(q, base, share);
+}
+
+// The CTA's groups folded over their R copies (R consecutive lanes per group) and
 // added to the HBM table. CTAs start at different groups, as smem_table_flush.
 template <int NA>
 __device__ __forceinline__ void lc_flush(const Plan& P, const unsigned long long* keys, const unsigned long long* acc,
-                                         Credit& cr) {
+                                         int S, int R, Credit* cr) {
   const LayoutAcc ly{P.L};
   const Layout& L = P.L;
-  const int kw = L.key_words, aw = P.smem_sw, R = P.smem_rep, S2 = P.smem_slots + 2;
+  const int kw = L.key_words, aw = P.smem_sw, S2 = S + 2;
   const int lane = threadIdx.x & 31, per = 32 / R, copy = lane & (R - 1);
   const int step = (int)(blockDim.x >> 5) * per;
   const int off0 = (int)(((long long)blockIdx.x * S2) / max(1, (int)gridDim.x));
@@ -525,7 +659,6 @@ __device__ __forceinline__ void lc_flush(const Plan& P, const unsigned long long
       }
     }
     if (copy != 0 || !have || rows == 0) continue;
-    const int S = P.smem_slots;
     unsigned long long k0 = 0, k1 = 0;
     const bool knull = kw > 0 && i == S + 1;
     if (kw > 0 && !knull) {
@@ -533,45 +666,26 @@ __device__ __forceinline__ void lc_flush(const Plan& P, const unsigned long long
       else if (P.gdense) k0 = (unsigned long long)P.gmin + (unsigned long long)i;
       else { k0 = keys[(size_t)i * kw]; if (kw == 2) k1 = keys[(size_t)i * 2 + 1]; }
     }
-    unsigned long long* g = find_global(ly, P.T, k0, k1, knull, P.err, &cr);
+    unsigned long long* g = find_global(ly, P.T, k0, k1, knull, P.err, cr);
     if (g != nullptr) apply<NA, false>(ly, g, c, rows);
   }
 }
 
-// SH: groups in the CTA's shared memory; otherwise in the launch's key window
-// (wg_window.cuh), nothing when it has none.
-template <int NA, bool SH>
-__global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_constant__ Plan P) {
-  extern __shared__ __align__(16) unsigned long long sm[];
-  __shared__ int s_groups;
-  __shared__ unsigned long long s_init[WG_MAX_SLOT_WORDS];
-  KeyWindow win;
-  win.base = 0;
-  win.n = 0;
-  if (!SH) {
-    win = *P.win;
-    if (win.n == 0) return;
-  }
-  const int S = P.smem_slots, kw = P.L.key_words, aw = P.smem_sw, R = P.smem_rep;
-  const int key_words = P.gdense ? 0 : S * kw;
-  unsigned long long* keys = sm;
-  unsigned long long* acc = sm + key_words;
-  const int s_limit = (S * 7) / 8;
-  if (SH) {
-    if (threadIdx.x < (unsigned)P.L.slot_words) s_init[threadIdx.x] = P.L.init[threadIdx.x];
-    if (threadIdx.x == 0) s_groups = 0;
-    for (int i = threadIdx.x; i < key_words; i += blockDim.x) keys[i] = kw == 1 ? WG_EMPTY_KEY : ~0ULL;
-    __syncthreads();
-    fill_pattern(acc, (int64_t)R * (S + 2) * aw, aw, P.L.slot_words - kw, s_init + kw, threadIdx.x, blockDim.x);
-    __syncthreads();
-  }
-  Credit cr;
+// The rows of the warp from base on. SH: groups in the CTA's shared memory, S slots
+// at sm and the copy of the accumulators that the lane adds to at mine; otherwise
+// in the key window win, its accumulators at mine. REST: after the CTA's second layout.
+// Returns the row at which the warp stopped: the end of the input, or where its CTA
+// is to change the layout.
+template <int NA, bool SH, bool REST>
+__device__ __forceinline__ int64_t lc_rows(const Plan& P, const KeyWindow& win, unsigned long long* sm, int S,
+                                           unsigned long long* mine, int64_t base, FarQueue* queue, volatile int* s_quit,
+                                           Credit* cr) {
   const int lane = threadIdx.x & 31;
-  unsigned long long* mine = SH ? acc + (size_t)(lane & (R - 1)) * (S + 2) * aw : P.wslots + kw;
   const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * (32 * kLcRows);
   const int jt = P.has_join ? (P.join.direct ? WG_JOIN_INNER : P.join.jtype) : WG_JOIN_INNER;
-  for (int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * kLcRows); base < P.n_items;
-       base += step) {
+  bool look = !REST || S > 0;  // for shared slots
+  for (; base < P.n_items; base += step) {
+    bool quit = false;
     LcRowSet r;
     r.base = P.sel ? 0 : base;
     unsigned live = 0;
@@ -606,12 +720,25 @@ __global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_con
       LcExprs ev;
 #pragma unroll 1
       for (int e = 0; e < P.n_exprs; ++e) lc_eval(P, r, e, live, ev.v + e * kLcRows, ev.null[e]);
-      int slot[kLcRows];
-      unsigned far;
-      const unsigned have = lc_keys<SH>(P, win, r, ev, live, keys, slot, far, &s_groups, s_limit);
-      lc_update<SH>(P, r, ev, have, mine, slot);
-      if (far) {
-        WG_LC_LIVE(u, far) lc_far_row(P, r.row(u), r.brow[u], &cr);
+      unsigned far = live;
+      if (!REST || look) {
+        int slot[kLcRows];
+        const unsigned have = lc_keys<SH>(P, win, r, ev, live, sm, S, slot, far);
+        lc_update<SH>(P, r, ev, have, mine, slot);
+      }
+      if (__any_sync(WG_FULL_MASK, far != 0)) {
+        // Another layout holds more groups. Where there is none (left), a row without a slot has cost
+        // the probes on top of its way through the HBM table: 2^24 rows into 1000 groups with a fifth
+        // of them without took 1.8 ms, all of them 1.35.
+        const int share = !SH || (P.gdense && !REST) ? 0 : !REST && P.smem_more > 0 ? 16 : 6;
+        const bool many = far_rows<DynShape, kLcRows, true>(P, queue, far, cr, r.row(0), r.row(1), r.brow[0], r.brow[1], base, share);
+        if (REST) {
+          look = look && !many;
+        } else if (SH) {
+          if (many) *s_quit = 1;
+          __syncwarp();
+          quit = __any_sync(WG_FULL_MASK, *s_quit != 0);
+        }
       }
       if (!chained) break;  // at most one match per row
       live = 0;             // arenaNext chain (join.go:2700)
@@ -620,11 +747,70 @@ __global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_con
         live |= nxt[u] >= 0 ? 1u << u : 0u;
       }
     }
+    if (SH && !REST && quit) return base + step;
   }
+  return base;
+}
+
+__device__ __forceinline__ void lc_init(const Plan& P, unsigned long long* sm, int S, int R, const unsigned long long* init) {
+  const int kw = P.L.key_words, key_words = P.gdense ? 0 : S * kw;
+  for (int i = threadIdx.x; i < key_words; i += blockDim.x) sm[i] = kw == 1 ? WG_EMPTY_KEY : ~0ULL;
+  __syncthreads();
+  fill_pattern(sm + key_words, (int64_t)R * (S + 2) * P.smem_sw, P.smem_sw, P.L.slot_words - kw, init + kw, threadIdx.x, blockDim.x);
+  __syncthreads();
+}
+
+// The rest of a CTA's rows with P.smem_more slots of one copy, none where that is 0.
+template <int NA>
+static __device__ __noinline__ void lc_rest(const Plan& P, unsigned long long* sm, const unsigned long long* init, int64_t base,
+                                            FarQueue* queue, Credit* cr) {
+  const int S = P.smem_more;
+  unsigned long long* acc = sm + S * P.L.key_words;
+  if (S > 0) lc_init(P, sm, S, 1, init);
+  queue->far = 0;
+  queue->mark = 128;
+  queue->from = base;
+  lc_rows<NA, true, true>(P, KeyWindow{0, 0}, sm, S, acc, base, queue, nullptr, cr);
+  __syncthreads();
+  if (S > 0) lc_flush<NA>(P, sm, acc, S, 1, cr);
+}
+
+// SH: groups in the CTA's shared memory; otherwise in the launch's key window
+// (wg_window.cuh), nothing when it has none.
+template <int NA, bool SH>
+__global__ void __launch_bounds__(kLcThreads, 1) lowcard_kernel(const __grid_constant__ Plan P) {
+  extern __shared__ __align__(16) unsigned long long sm[];
+  __shared__ int s_quit;
+  __shared__ unsigned long long s_init[WG_MAX_SLOT_WORDS];
+  KeyWindow win;
+  win.base = 0;
+  win.n = 0;
+  if (!SH) {
+    win = *P.win;
+    if (win.n == 0) return;
+  }
+  Credit cr;
+  int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * kLcRows);
+  FarQueue queue;
+  far_init(queue, base);
   if (SH) {
+    const int S = P.smem_slots, R = P.smem_rep;
+    unsigned long long* acc = sm + (P.gdense ? 0 : S * P.L.key_words);
+    if (threadIdx.x < (unsigned)P.L.slot_words) s_init[threadIdx.x] = P.L.init[threadIdx.x];
+    if (threadIdx.x == 0) s_quit = 0;
+    lc_init(P, sm, S, R, s_init);
+    unsigned long long* mine = acc + (size_t)(threadIdx.x & (unsigned)(R - 1)) * (S + 2) * P.smem_sw;
+    base = lc_rows<NA, true, false>(P, win, sm, S, mine, base, &queue, &s_quit, &cr);
     __syncthreads();
-    lc_flush<NA>(P, keys, acc, cr);
+    lc_flush<NA>(P, sm, acc, S, R, &cr);
+    if (s_quit) {
+      __syncthreads();  // the table is read before it is laid out anew
+      lc_rest<NA>(P, sm, s_init, base, &queue, &cr);
+    }
+  } else {
+    lc_rows<NA, false, false>(P, win, sm, 0, P.wslots + P.L.key_words, base, &queue, nullptr, &cr);
   }
+  far_flush<DynShape>(P, &queue, &cr);
   cr.release(P.T);
 }
 

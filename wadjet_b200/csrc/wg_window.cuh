@@ -129,6 +129,8 @@ __global__ void __launch_bounds__(kWinBlock, 2) window_group_kernel(const __grid
   const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5) * (32 * U);
   int64_t base = ((int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5)) * (32 * U);
   const bool test = P.minmax_test != 0;
+  FarQueue queue;
+  far_init(queue, base);
   for (;;) {
     unsigned far = 0;
     for (; base < P.n_items; base += step) {
@@ -152,9 +154,10 @@ __global__ void __launch_bounds__(kWinBlock, 2) window_group_kernel(const __grid
       if (__any_sync(WG_FULL_MASK, far != 0)) break;
     }
     if (base >= P.n_items) break;
-    for (; far; far &= far - 1) lc_far_row(P, base + (int64_t)lane * U + __ffs(far) - 1, -1, &cr);
+    far_rows<StatShape<C>, U, false>(P, &queue, far, &cr, base + (int64_t)lane * U);
     base += step;
   }
+  far_flush<StatShape<C>>(P, &queue, &cr);
   cr.release(P.T);
 }
 
