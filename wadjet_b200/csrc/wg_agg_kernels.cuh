@@ -154,6 +154,8 @@ template <class C>
 struct StatShape {
   static constexpr bool smem_ok = C::smem_ok;
   static constexpr int kAggs = C::n_aggs;
+  // the vector kernels with a shared table: shapes without a join have lean_group_kernel
+  static constexpr bool vec_smem = C::smem_ok && C::has_join != 0;
   // straight-line code fits 40 registers: two 768-thread CTAs per SM (48 warps)
   static constexpr int kBlock = 768, kMinBlocks = 2;
   // vector kernel: evaluate all of a lane's rows before their table updates

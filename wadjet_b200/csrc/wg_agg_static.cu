@@ -51,7 +51,7 @@ static void launch_lean_t(const LaunchSpec& l, unsigned block, cudaStream_t st) 
 
 template <class C>
 static bool launch_lean(const LaunchSpec& ls, cudaStream_t st) {
-  if (ls.vec == 0 || !ls.smem || ls.tile || ls.stage || ls.P.gdense || ls.P.smem_combine) return false;
+  if (ls.vec == 0 || !ls.smem || ls.tile) return false;
   LaunchSpec l = ls;
   const bool whole = ls.block == 1024;  // the table takes a whole SM
   constexpr bool any_float = wgd::lean_float_sums<C>() > 0;

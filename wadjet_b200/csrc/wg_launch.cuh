@@ -63,7 +63,7 @@ static void launch_vec_t(const LaunchSpec& ls, cudaStream_t st, bool smem) {
   if constexpr (std::is_same<Sh, wgd::DynShape>::value) {
     (void)ls; (void)st; (void)smem;
   } else {
-    if constexpr (Sh::smem_ok) {
+    if constexpr (Sh::vec_smem) {
       if (smem && ls.stage) { launch_stage_one<NA, Sh>(ls, st); return; }
       if (smem) { launch_vec_s<NA, Sh, true>(ls, st); return; }
     }

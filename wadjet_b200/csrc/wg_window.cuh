@@ -6,8 +6,8 @@
 // else waits for, a warp-wide match for rows of one group, and then an L2 atomic per
 // sum. Identifiers, codes, prefixes and string ids mostly come from a range
 // not much wider than their distinct count: then the slot is an offset, nothing is read
-// before the updates, and the bound is the L2 atomics (about 190 G/s on
-// this part: 10^8 rows into 65536 groups, a sum and a count, 1251 us of atomics against
+// before the updates, and the bound is the L2 atomics (10^8 rows into 65536 groups, a sum
+// and a count each: 1228 us, 163 G atomics/s of the 190 measured at most, against
 // 2262 us through the hash table; 2 * 10^7 rows of string ids into 10^5 groups 342
 // against 869 us).
 //
