@@ -472,7 +472,9 @@ __device__ __forceinline__ bool f64_to_fixed_scaled(double d, double scale, unsi
   const long long q = __double2ll_rn(y);
   lo = (unsigned long long)q;
   hi = (unsigned long long)(q >> 63);
-  return fabs(y) < 0x1p62 && __ll2double_rn(q) == y && q != 0;
+  // the exponent field in [1, 1085): a normal number (not 0, nor what underflowed to it) below 2^62
+  const unsigned e = (unsigned)__double2hiint(y) << 1;
+  return e - (1u << 21) < (1084u << 21) && __ll2double_rn(q) == y;
 }
 
 // (the exponent field of the largest value; 2^e stays a normal number)
