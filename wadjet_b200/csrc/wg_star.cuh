@@ -25,7 +25,8 @@
 //
 // What bounds it at 2^28 fact rows: 1939 us with the float SUM as four lane-striped float64
 // copies, 1546 without that SUM, 1482 without any table update, 1317 the copy
-// peak's time for its bytes; the two 32-bit limb adds bring it to 1688 us.
+// peak's time for its bytes; the two 32-bit limb adds bring it to about 1700 us (1688 to
+// 1733 over three boxes).
 #pragma once
 
 #include "wg_shapes.cuh"
