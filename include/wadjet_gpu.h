@@ -227,7 +227,8 @@ WG_API wg_status wg_ctx_create_child(wg_ctx* parent, wg_ctx** out);
 WG_API wg_status wg_ctx_destroy(wg_ctx* ctx);
 /* Wait until all work queued on the context's stream is done. */
 WG_API wg_status wg_ctx_synchronize(wg_ctx* ctx);
-/* Ledger counters (Tracker.Used / Peak / Budget, tracker.go:129,151,134). */
+/* Ledger counters (Tracker.Used / Peak / Budget, tracker.go:129,151,134). Blocks that the
+ * context keeps for its next call count as used until a reservation needs them. */
 WG_API wg_status wg_ledger_stats(wg_ctx* ctx, int64_t* used, int64_t* peak, int64_t* budget);
 /* Explicit reservations against the ledger (Tracker.Reserve/Release,
  * tracker.go:53,73); WG_E_NOMEM when over budget, nothing reserved then. */
